@@ -2,8 +2,8 @@
 //
 // Everything a ray touches in its inner loop is 16-byte aligned and read with
 // 128-bit loads:
-//   DevNode      64 B  both children's boxes of one interior node of the
-//                      reference's binary SAH BVH (same topology, child-box form)
+//   DevNode     128 B  the four child boxes of two collapsed levels of the
+//                      reference's binary SAH BVH
 //   DevTriangle  48 B  three vertices of one triangle, in BVH leaf order
 //   DevObject    16 B  one TLAS primitive (sphere, triangle or instance), leaf order
 //   DevSphere    16 B  center and radius
@@ -28,10 +28,11 @@ constexpr std::uint32_t kMaxLeafFirst{kLeafFirstMask};
 
 // A 4-wide node: two levels of the reference's binary BVH collapsed into one.
 // Child i's box is (lo_x[i], hi_x[i], lo_y[i], ...); absent children are
-// kEmptyChild. `order[o]` lists, for the ray octant o (bit a set when the
-// direction's component a is negative), the children in the order the
-// reference's depth-first, near-first traversal reaches them: 2 bits per child,
-// nearest first, low bits first.
+// kEmptyChild. `place[o]` gives, for the ray octant o (bit a set when the
+// direction's component a is negative), each child's place in the order the
+// reference's depth-first, near-first traversal reaches them, 0 first: bits 2c
+// and 2c + 1 for child c. The places are a permutation of 0..3; absent children
+// take the last ones.
 struct alignas(16) DevNode {
     float lo_x[4];
     float hi_x[4];
@@ -40,7 +41,7 @@ struct alignas(16) DevNode {
     float lo_z[4];
     float hi_z[4];
     std::uint32_t child[4];
-    std::uint8_t order[8];
+    std::uint8_t place[8];
     std::uint32_t count;  // children present (1..4); they are child[0..count-1]
     std::uint32_t groups; // slots per binary child of the collapsed node (bits 0-1, 2-3); 0 for a leaf root
 };

@@ -118,6 +118,7 @@ Emitted emitBvh(const BuiltBvh& bvh, std::uint64_t prim_base, std::vector<DevNod
             setChildBox(dev, 0, bvh.nodes[i].bounds);
             dev.child[0] = leafRef(prim_base + bvh.nodes[i].offset, bvh.nodes[i].count);
             dev.count = 1;
+            std::fill(std::begin(dev.place), std::end(dev.place), std::uint8_t{0xE4});
             continue;
         }
         // Groups: the first and second child of i, each a leaf or two children.
@@ -148,19 +149,21 @@ Emitted emitBvh(const BuiltBvh& bvh, std::uint64_t prim_base, std::vector<DevNod
         dev.groups = static_cast<std::uint32_t>(groups[0].size) | (static_cast<std::uint32_t>(groups[1].size) << 2U);
         for (unsigned octant{0}; octant < 8; ++octant) {
             const bool swap{((octant >> bvh.nodes[i].axis) & 1U) != 0};
-            std::uint8_t packed{0};
-            int position{0};
+            // Absent children, slots count..3, take the last places.
+            unsigned packed{0xE4U & ~((1U << (2 * dev.count)) - 1U)};
+            unsigned position{0};
+            const auto placeNext = [&](int slot_index) { packed |= position++ << (2 * slot_index); };
             for (int g{0}; g < 2; ++g) {
                 const Group& group{groups[swap ? 1 - g : g]};
                 if (group.size == 1) {
-                    packed |= static_cast<std::uint8_t>(group.first_slot << (2 * position++));
+                    placeNext(group.first_slot);
                 } else {
                     const bool inner_swap{((octant >> bvh.nodes[group.node].axis) & 1U) != 0};
-                    packed |= static_cast<std::uint8_t>((group.first_slot + (inner_swap ? 1 : 0)) << (2 * position++));
-                    packed |= static_cast<std::uint8_t>((group.first_slot + (inner_swap ? 0 : 1)) << (2 * position++));
+                    placeNext(group.first_slot + (inner_swap ? 1 : 0));
+                    placeNext(group.first_slot + (inner_swap ? 0 : 1));
                 }
             }
-            dev.order[octant] = packed;
+            dev.place[octant] = static_cast<std::uint8_t>(packed);
         }
         // Stack need: pushes here (count - 1) plus the deepest interior child's need.
         std::uint32_t child_need{0};

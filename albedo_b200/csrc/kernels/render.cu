@@ -4,7 +4,8 @@
 // and draws its n x n stratified samples from it in row-major order, so one
 // thread runs one pixel's samples serially. Blocks cover tiles of 128 pixels
 // (16 x 8 by default) so a warp's camera rays start coherent. The traversal stack of every thread sits in
-// shared memory (STACK entries of 8 bytes).
+// shared memory: STACK child references of 4 bytes, or STACK entries of 8 bytes
+// in the counting kernels.
 #include "estimator.cuh"
 
 #include <type_traits>
@@ -13,7 +14,7 @@ namespace albedo_b200 {
 
 namespace {
 
-constexpr int kBlock = 128;
+constexpr int kBlock = kTraceBlock;
 constexpr int kTileW = 16; // default tile: 16 x 8 pixels
 // Resident blocks per SM the megakernel's register budget is sized for by
 // default: 3 (168 registers a thread) measured 4-12% faster than 4 (128
@@ -75,17 +76,18 @@ struct alignas(4) SharedPath {
 };
 static_assert(sizeof(SharedPath) % 8 == 4, "odd word stride");
 
-// Stack entry type of a megakernel variant: LEAN kernels keep the child
-// reference alone (4 bytes).
-template <bool LEAN>
-using MegaStackEntry = std::conditional_t<LEAN, unsigned, uint2>;
+// Stack entry type: the child reference alone (4 bytes), but for the counting
+// kernels, whose counts are those of a traversal that drops popped entries
+// beyond the current hit (8 bytes: reference and entry distance).
+template <bool COUNT>
+using StackEntry = std::conditional_t<COUNT, uint2, unsigned>;
 
 // INL: 0 = both queries call the shared out-of-line traversal, 1 = both are
 // inlined, 2 = the closest-hit query is inlined and the shadow query calls the
 // out-of-line copy (a smaller kernel than 1, no register saves around the
 // per-bounce call). LEAN: the path's state between bounces lives in shared
-// memory rather than registers and the stack entries are 4 bytes, so fewer
-// registers carry state across the traversal and more blocks fit an SM.
+// memory rather than registers, so fewer registers carry state across the
+// traversal and more blocks fit an SM.
 template <int STACK, int EST, bool COUNT = false, int MINB = kMegaBlocksPerSm, int ACC = kAccumulateFp64,
           int INL = 0, bool LEAN = false>
 __global__ void __launch_bounds__(kBlock, MINB) megakernel(const DevScene scene, const DevCamera camera,
@@ -93,12 +95,12 @@ __global__ void __launch_bounds__(kBlock, MINB) megakernel(const DevScene scene,
                                                           unsigned int* error_flag,
                                                           unsigned long long* totals = nullptr)
 {
-    using Entry = MegaStackEntry<LEAN>;
+    using Entry = StackEntry<COUNT>;
     extern __shared__ uint2 stack_memory[];
     Entry* const stack = reinterpret_cast<Entry*>(stack_memory);
     TraversalCounts counts{0, 0, 0, 0, 0, 0};
-    const TraceContext<INL != 0, COUNT, INL == 1, Entry> ctx{stack + threadIdx.x, kBlock, STACK, error_flag,
-                                                             COUNT ? &counts : nullptr};
+    const TraceContext<INL != 0, COUNT, INL == 1, Entry> ctx{TraceStack<Entry>::of(stack + threadIdx.x, STACK),
+                                                             error_flag, COUNT ? &counts : nullptr};
     int x, y, slot;
     if (args.pixels != nullptr) {
         slot = blockIdx.x * kBlock + threadIdx.x;
@@ -194,7 +196,8 @@ __global__ void __launch_bounds__(kBlock) traceCountKernel(const DevScene scene,
     TraceHit hit;
     float tmax = t_max;
     static_cast<void>(traceScene<false, false, true>(scene, o, d, t_min, tmax, SkipRule::none(), hit,
-                                                     stack + threadIdx.x, kBlock, STACK, error_flag, &counts));
+                                                     TraceStack<uint2>::of(stack + threadIdx.x, STACK), error_flag,
+                                                     &counts));
     atomicAdd(totals + 0, counts.boxes);
     atomicAdd(totals + 1, counts.triangles);
     atomicAdd(totals + 2, counts.spheres);
@@ -207,7 +210,7 @@ template <int STACK>
 __global__ void __launch_bounds__(kBlock) traceKernel(const DevScene scene, const float* rays, int count, float t_min,
                                                       float t_max, TraceOutputs out, unsigned int* error_flag)
 {
-    extern __shared__ uint2 stack[];
+    extern __shared__ unsigned ref_stack[];
     const int i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= count) {
         return;
@@ -216,8 +219,8 @@ __global__ void __launch_bounds__(kBlock) traceKernel(const DevScene scene, cons
     const float3 d = mk(rays[6 * i + 3], rays[6 * i + 4], rays[6 * i + 5]);
     TraceHit hit;
     float tmax = t_max;
-    const bool found = traceScene<false>(scene, o, d, t_min, tmax, SkipRule::none(), hit, stack + threadIdx.x, kBlock,
-                                         STACK, error_flag);
+    const bool found = traceScene<false>(scene, o, d, t_min, tmax, SkipRule::none(), hit,
+                                         TraceStack<unsigned>::of(ref_stack + threadIdx.x, STACK), error_flag);
     out.hit[i] = found ? 1 : 0;
     if (!found) {
         return;
@@ -249,7 +252,7 @@ template <int STACK>
 __global__ void __launch_bounds__(kBlock) occludedKernel(const DevScene scene, const float* rays, const float* t_max,
                                                          int count, int* occluded_out, unsigned int* error_flag)
 {
-    extern __shared__ uint2 stack[];
+    extern __shared__ unsigned ref_stack[];
     const int i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= count) {
         return;
@@ -258,16 +261,18 @@ __global__ void __launch_bounds__(kBlock) occludedKernel(const DevScene scene, c
     const float3 d = mk(rays[6 * i + 3], rays[6 * i + 4], rays[6 * i + 5]);
     TraceHit hit;
     float tmax = t_max[i];
-    occluded_out[i] = traceScene<true>(scene, o, d, 0.0f, tmax, SkipRule::none(), hit, stack + threadIdx.x, kBlock,
-                                       STACK, error_flag)
+    occluded_out[i] = traceScene<true>(scene, o, d, 0.0f, tmax, SkipRule::none(), hit,
+                                       TraceStack<unsigned>::of(ref_stack + threadIdx.x, STACK), error_flag)
                           ? 1
                           : 0;
 }
 
-constexpr std::size_t stackBytes(int stack, std::size_t entry_bytes = sizeof(uint2))
+constexpr std::size_t stackBytes(int stack, std::size_t entry_bytes)
 {
     return static_cast<std::size_t>(stack) * kBlock * entry_bytes;
 }
+
+constexpr int kCountEntry = static_cast<int>(sizeof(StackEntry<true>));
 
 int megaBlocks(const RenderArgs& args)
 {
@@ -281,7 +286,7 @@ int megaBlocks(const RenderArgs& args)
 
 // Launches `kernel` over `blocks` blocks with a STACK-entry shared-memory stack
 // of ENTRY-byte entries.
-template <int STACK, int ENTRY = static_cast<int>(sizeof(uint2)), typename Kernel, typename... Args>
+template <int STACK, int ENTRY = static_cast<int>(sizeof(unsigned)), typename Kernel, typename... Args>
 cudaError_t launchStacked(Kernel kernel, int blocks, cudaStream_t stream, Args... args)
 {
     if (blocks == 0) {
@@ -303,7 +308,7 @@ cudaError_t launchMegakernelCounting(const DevScene& scene, const DevCamera& cam
 {
     return withStack(stack_capacity, [&](auto size) {
         constexpr int S = decltype(size)::value;
-        return launchStacked<S>(megakernel<S, kEstimatorPath, true>, megaBlocks(args), stream, scene, camera, args,
+        return launchStacked<S, kCountEntry>(megakernel<S, kEstimatorPath, true>, megaBlocks(args), stream, scene, camera, args,
                                 accum, error_flag, totals);
     });
 }
@@ -323,8 +328,7 @@ int stackCapacityFor(std::uint32_t stack_need)
 }
 
 // Path-estimator megakernel of the shape `args` names: blocks_per_sm 3 (state
-// in registers, 8-byte stack entries) or 4 (lean: state in shared memory,
-// 4-byte stack entries), and how its traversal is placed (inline_traversal).
+// in registers) or 4 (lean: state in shared memory), and how its traversal is placed (inline_traversal).
 template <int S, int ACC>
 cudaError_t launchPathMegakernel(const DevScene& scene, const DevCamera& camera, const RenderArgs& args,
                                  PixelAccum* accum, unsigned int* error_flag, cudaStream_t stream)
@@ -332,12 +336,11 @@ cudaError_t launchPathMegakernel(const DevScene& scene, const DevCamera& camera,
     unsigned long long* no_totals = nullptr;
     const int blocks = megaBlocks(args);
     if (args.blocks_per_sm == 4) {
-        constexpr int kEntry = static_cast<int>(sizeof(unsigned));
         if (args.inline_traversal == 1) {
-            return launchStacked<S, kEntry>(megakernel<S, kEstimatorPath, false, 4, ACC, 1, true>, blocks, stream,
+            return launchStacked<S>(megakernel<S, kEstimatorPath, false, 4, ACC, 1, true>, blocks, stream,
                                             scene, camera, args, accum, error_flag, no_totals);
         }
-        return launchStacked<S, kEntry>(megakernel<S, kEstimatorPath, false, 4, ACC, 0, true>, blocks, stream, scene,
+        return launchStacked<S>(megakernel<S, kEstimatorPath, false, 4, ACC, 0, true>, blocks, stream, scene,
                                         camera, args, accum, error_flag, no_totals);
     }
     if (args.inline_traversal == 1) {
@@ -390,7 +393,7 @@ cudaError_t launchTraceCounting(const DevScene& scene, const float* rays, int co
 {
     return withStack(stack_capacity, [&](auto size) {
         constexpr int S = decltype(size)::value;
-        return launchStacked<S>(traceCountKernel<S>, (count + kBlock - 1) / kBlock, stream, scene, rays, count, t_min,
+        return launchStacked<S, kCountEntry>(traceCountKernel<S>, (count + kBlock - 1) / kBlock, stream, scene, rays, count, t_min,
                                 t_max, error_flag, totals);
     });
 }

@@ -12,14 +12,19 @@
 // outward, which can only add box hits, never lose one.
 //
 // The traversal stack lives in shared memory: entry i of thread `lane` is at
-// stack[i * stride + lane] (entry-major, so a warp touching the same depth hits
-// consecutive banks). An entry is either (child reference, entry distance), 8
-// bytes, and a popped entry whose box is entered beyond the current hit is
-// dropped as the reference drops it; or the child reference alone, 4 bytes,
-// and the popped node or leaf is visited and culled by its own box tests. Both
-// give the same hits: a primitive below a node entered beyond the current hit
-// cannot be hit nearer than it. The 4-byte form halves the shared memory of
-// the wavefront's persistent traversal kernels, so more of them fit on an SM.
+// stack[i * 128 + lane] (entry-major, so a warp touching the same depth hits
+// consecutive banks). An entry is the child reference alone, 4 bytes, and the
+// popped node or leaf is visited and culled by its own tests; or (child
+// reference, entry distance), 8 bytes, and a popped entry whose box is entered
+// beyond the current hit is dropped as the reference drops it. Both give the
+// same hits: a primitive below a node entered beyond the current hit cannot be
+// hit nearer than it. Every timed kernel uses the 4-byte form: the drop loop of
+// the 8-byte form splits a warp's lanes further (megakernel at 3 blocks per SM:
+// 1.31M-triangle icosphere at 1920x1080, 36 samples, 419.8 ms with 8-byte
+// entries and 215.7 with 4-byte; 200,003-triangle soup at 853x481, 16 samples,
+// 148.0 and 63.2; instanced trefoils at 960x540, 64 samples, 383.7 and 322.3),
+// and it halves the shared memory. The counting kernels keep the 8-byte form,
+// whose counts are the reference's.
 #pragma once
 
 #include "common.cuh"
@@ -354,7 +359,7 @@ ALB_DEV std::uint32_t leafRef(std::uint32_t first, std::uint32_t count)
 
 // One ray query in flight: the ray in the space being traversed (world or the
 // current instance's object space), the world ray it came from, the live range,
-// the node reference to visit next, the stack depth and the hit so far.
+// the node reference to visit next, the stack's top and the hit so far.
 struct TraceState {
     TravRay r;
     float3 origin;
@@ -363,7 +368,7 @@ struct TraceState {
     float tmax;
     std::uint32_t ref;
     std::uint32_t inst_pos; // TLAS leaf position of the instance being traversed, or kNoPrim
-    int sp;
+    unsigned sp; // shared address of the next free stack entry
     bool found;
     // The ray changes space (entering or leaving an instance): r.o and r.inv
     // hold the new origin and direction, and the next step sets the ray up from
@@ -394,7 +399,8 @@ enum TraceStep : int {
 };
 
 // Starts a query over (tmin, tmax); false when the scene has no objects.
-ALB_DEV bool traceBegin(const DevScene& s, TraceState& q, float3 origin, float3 dir, float tmin, float tmax)
+ALB_DEV bool traceBegin(const DevScene& s, TraceState& q, unsigned stack_base, float3 origin, float3 dir, float tmin,
+                        float tmax)
 {
     q.origin = origin;
     q.dir = dir;
@@ -402,7 +408,7 @@ ALB_DEV bool traceBegin(const DevScene& s, TraceState& q, float3 origin, float3 
     q.tmax = tmax;
     q.found = false;
     q.resetup = false;
-    q.sp = 0;
+    q.sp = stack_base;
     q.inst_pos = kNoPrim;
     q.ref = s.tlas_root;
     if (s.tlas_root == kEmptyChild) {
@@ -448,22 +454,60 @@ __device__ __forceinline__ void countReferenceBoxes(const float4& lx, const floa
     }
 }
 
+// A thread's traversal stack, by its shared-memory address: entry i is kStride
+// bytes above entry i - 1 (entries of one depth are adjacent across the block's
+// 128 threads). Entries are read and written with shared-memory instructions: a
+// store through a generic pointer could alias any table, and the compiler then
+// reloads the scene's table addresses after every push.
+constexpr int kTraceBlock = 128;
+
+template <typename Entry>
+struct TraceStack {
+    static constexpr unsigned kStride = kTraceBlock * sizeof(Entry);
+    unsigned base; // entry 0
+    unsigned end;  // one past the last entry
+
+    // `stack` is the block's stack memory at this thread's entry 0.
+    ALB_DEV static TraceStack of(Entry* stack, int entries)
+    {
+        const unsigned base = static_cast<unsigned>(__cvta_generic_to_shared(stack));
+        return {base, base + static_cast<unsigned>(entries) * kStride};
+    }
+};
+
 // One stack entry: child reference and entry distance, or the reference alone.
-__device__ __forceinline__ void pushEntry(uint2* slot, std::uint32_t ref, float entry)
+ALB_DEV void pushEntry(const TraceStack<uint2>&, unsigned at, std::uint32_t ref, float entry)
 {
-    *slot = make_uint2(ref, __float_as_uint(entry));
+    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at), "r"(ref), "r"(__float_as_uint(entry)));
 }
-__device__ __forceinline__ void pushEntry(unsigned* slot, std::uint32_t ref, float)
+ALB_DEV void pushEntry(const TraceStack<unsigned>&, unsigned at, std::uint32_t ref, float)
 {
-    *slot = ref;
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(ref));
+}
+ALB_DEV uint2 loadEntry(const TraceStack<uint2>&, unsigned at)
+{
+    uint2 e;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(e.x), "=r"(e.y) : "r"(at));
+    return e;
+}
+ALB_DEV unsigned loadEntry(const TraceStack<unsigned>&, unsigned at)
+{
+    unsigned e;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(e) : "r"(at));
+    return e;
 }
 
 // A 4-wide node: tests every child box, continues with the hit child the
 // reference reaches first and pushes the other hit children, last first, so
 // leaves are reached in the reference's depth-first near-first order.
+//
+// Without branches: child c's place p_c in the order comes from the node's
+// per-octant table, the hit children set bits p_c of `hits`, the lowest set bit
+// is the next child and a child's entry lies above the entries of the set bits
+// beyond its own.
 template <typename Stack>
-__device__ __forceinline__ int nodeStep(const DevNode* nodes, TraceState& q, Stack* stack, int stride,
-                                        int stack_size, unsigned int* error_flag, TraversalCounts* counts)
+__device__ __forceinline__ int nodeStep(const DevNode* nodes, TraceState& q, const Stack& stack,
+                                        unsigned int* error_flag, TraversalCounts* counts)
 {
     const float4* np = reinterpret_cast<const float4*>(nodes + q.ref);
     const uint4 ch = __ldg(reinterpret_cast<const uint4*>(np + 6));
@@ -475,54 +519,56 @@ __device__ __forceinline__ int nodeStep(const DevNode* nodes, TraceState& q, Sta
         countReferenceBoxes(__ldg(np), __ldg(np + 1), __ldg(np + 2), __ldg(np + 3), __ldg(np + 4), __ldg(np + 5),
                             meta.w, r, q.tmin, q.tmax, *counts);
     }
-    float e0 = 0.0f, e1 = 0.0f, e2 = 0.0f, e3 = 0.0f;
-    unsigned mask;
-    {
-        // Near and far planes per axis by the sign of the inverse direction:
-        // axis a's lo array is np[2a], its hi array np[2a + 1].
-        const unsigned sx = r.planes & 1u;
-        const unsigned sy = (r.planes >> 1) & 1u;
-        const unsigned sz = (r.planes >> 2) & 1u;
-        const float4 nx = __ldg(np + sx);
-        const float4 fx = __ldg(np + (1u - sx));
-        const float4 ny = __ldg(np + 2u + sy);
-        const float4 fy = __ldg(np + (3u - sy));
-        const float4 nz = __ldg(np + 4u + sz);
-        const float4 fz = __ldg(np + (5u - sz));
-        mask = (slabTestOrdered(nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, r, q.tmin, q.tmax, e0) ? 1u : 0u) |
-               (slabTestOrdered(nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, r, q.tmin, q.tmax, e1) ? 2u : 0u) |
-               (slabTestOrdered(nx.z, fx.z, ny.z, fy.z, nz.z, fz.z, r, q.tmin, q.tmax, e2) ? 4u : 0u) |
-               (slabTestOrdered(nx.w, fx.w, ny.w, fy.w, nz.w, fz.w, r, q.tmin, q.tmax, e3) ? 8u : 0u);
-        // Absent children (zero boxes) are tested too and masked off here.
-        mask &= (1u << present) - 1u;
-    }
-    if (mask == 0u) {
+    // Near and far planes per axis by the sign of the inverse direction: axis
+    // a's lo array is np[2a], its hi array np[2a + 1].
+    const unsigned sx = r.planes & 1u;
+    const unsigned sy = (r.planes >> 1) & 1u;
+    const unsigned sz = (r.planes >> 2) & 1u;
+    const float4 nx = __ldg(np + sx);
+    const float4 fx = __ldg(np + (1u - sx));
+    const float4 ny = __ldg(np + 2u + sy);
+    const float4 fy = __ldg(np + (3u - sy));
+    const float4 nz = __ldg(np + 4u + sz);
+    const float4 fz = __ldg(np + (5u - sz));
+    float e0, e1, e2, e3;
+    const bool h0 = slabTestOrdered(nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, r, q.tmin, q.tmax, e0);
+    const bool h1 = slabTestOrdered(nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, r, q.tmin, q.tmax, e1);
+    const bool h2 = slabTestOrdered(nx.z, fx.z, ny.z, fy.z, nz.z, fz.z, r, q.tmin, q.tmax, e2);
+    const bool h3 = slabTestOrdered(nx.w, fx.w, ny.w, fy.w, nz.w, fz.w, r, q.tmin, q.tmax, e3);
+    // The octant's byte of the table; child c's place is its bits 2c, 2c + 1.
+    // Absent children (zero boxes) are tested too; their places lie beyond
+    // those of the children present and are masked off.
+    const unsigned places = __byte_perm(meta.x, meta.y, r.neg);
+    const unsigned b0 = 1u << (places & 3u);
+    const unsigned b1 = 1u << ((places >> 2) & 3u);
+    const unsigned b2 = 1u << ((places >> 4) & 3u);
+    const unsigned b3 = 1u << ((places >> 6) & 3u);
+    const unsigned hits =
+        ((h0 ? b0 : 0u) | (h1 ? b1 : 0u) | (h2 ? b2 : 0u) | (h3 ? b3 : 0u)) & ((1u << present) - 1u);
+    if (hits == 0u) {
         return kStepPop;
     }
-    int remaining = __popc(mask);
-    if (q.sp + remaining - 1 > stack_size) {
+    const unsigned first = hits & (0u - hits);
+    const unsigned pushed = hits ^ first;
+    const unsigned top = q.sp + static_cast<unsigned>(__popc(pushed)) * Stack::kStride;
+    if (top > stack.end) {
         atomicOr(error_flag, 1u);
         return kStepFinished;
     }
-    const unsigned packed = (r.neg < 4u ? (meta.x >> (8u * r.neg)) : (meta.y >> (8u * (r.neg - 4u)))) & 0xFFu;
-#pragma unroll
-    for (int position = 3; position >= 0; --position) {
-        if (position >= present) {
-            continue;
-        }
-        const unsigned c = (packed >> (2 * position)) & 3u;
-        if (((mask >> c) & 1u) == 0u) {
-            continue;
-        }
-        const std::uint32_t child = c == 0u ? ch.x : (c == 1u ? ch.y : (c == 2u ? ch.z : ch.w));
-        if (--remaining == 0) {
+    const auto take = [&](unsigned bit, std::uint32_t child, float entry) {
+        if ((first & bit) != 0u) {
             q.ref = child;
-        } else {
-            const float entry = c == 0u ? e0 : (c == 1u ? e1 : (c == 2u ? e2 : e3));
-            pushEntry(stack + q.sp * stride, child, entry);
-            ++q.sp;
         }
-    }
+        if ((pushed & bit) != 0u) {
+            pushEntry(stack, q.sp + static_cast<unsigned>(__popc(hits & (0u - (bit << 1)))) * Stack::kStride, child,
+                      entry);
+        }
+    };
+    take(b0, ch.x, e0);
+    take(b1, ch.y, e1);
+    take(b2, ch.z, e2);
+    take(b3, ch.w, e3);
+    q.sp = top;
     return kStepDescend;
 }
 
@@ -530,9 +576,8 @@ __device__ __forceinline__ int nodeStep(const DevNode* nodes, TraceState& q, Sta
 // instance is entered at once (the rest of the leaf and an exit marker are
 // pushed). In a BLAS: the current instance's triangles.
 template <typename Stack>
-__device__ __forceinline__ int leafStep(const DevScene& s, TraceState& q, const SkipRule& skip, Stack* stack,
-                                        int stride, int stack_size, unsigned int* error_flag,
-                                        TraversalCounts* counts, bool any)
+__device__ __forceinline__ int leafStep(const DevScene& s, TraceState& q, const SkipRule& skip, const Stack& stack,
+                                        unsigned int* error_flag, TraversalCounts* counts, bool any)
 {
     const std::uint32_t first = q.ref & kLeafFirstMask;
     const std::uint32_t count = ((q.ref >> 28) & 7u) + 1u;
@@ -551,16 +596,16 @@ __device__ __forceinline__ int leafStep(const DevScene& s, TraceState& q, const 
                 continue;
             }
             if (obj.kind == kObjInstance) {
-                if (q.sp + 2 > stack_size) {
+                if (q.sp + 2 * Stack::kStride > stack.end) {
                     atomicOr(error_flag, 1u);
                     return kStepFinished;
                 }
                 if (k + 1 < count) {
-                    pushEntry(stack + q.sp * stride, leafRef(pos + 1, count - k - 1), -INFINITY);
-                    ++q.sp;
+                    pushEntry(stack, q.sp, leafRef(pos + 1, count - k - 1), -INFINITY);
+                    q.sp += Stack::kStride;
                 }
-                pushEntry(stack + q.sp * stride, kExitMarker, 0.0f);
-                ++q.sp;
+                pushEntry(stack, q.sp, kExitMarker, 0.0f);
+                q.sp += Stack::kStride;
                 const DevInstance& inst = s.instances[obj.index];
                 if (counts != nullptr) {
                     counts->instances += 1;
@@ -613,14 +658,14 @@ __device__ __forceinline__ int leafStep(const DevScene& s, TraceState& q, const 
 // Pops the next entry still worth visiting into `ref`; false when none is left.
 // An exit marker returns the ray to world space; an entry whose box is entered
 // beyond the current hit is dropped (accel/bvh.hpp:240-247).
-__device__ __forceinline__ bool popNext(TraceState& q, const uint2* stack, int stride)
+__device__ __forceinline__ bool popNext(TraceState& q, const TraceStack<uint2>& stack)
 {
     for (;;) {
-        if (q.sp == 0) {
+        if (q.sp == stack.base) {
             return false;
         }
-        --q.sp;
-        const uint2 e = stack[q.sp * stride];
+        q.sp -= TraceStack<uint2>::kStride;
+        const uint2 e = loadEntry(stack, q.sp);
         if (e.x == kExitMarker) {
             q.changeSpace(q.origin, q.dir);
             q.inst_pos = kNoPrim;
@@ -636,14 +681,14 @@ __device__ __forceinline__ bool popNext(TraceState& q, const uint2* stack, int s
 
 // The same for 4-byte entries: no entry distance, so nothing is dropped here;
 // the popped node's or leaf's own tests cull it.
-__device__ __forceinline__ bool popNext(TraceState& q, const unsigned* stack, int stride)
+__device__ __forceinline__ bool popNext(TraceState& q, const TraceStack<unsigned>& stack)
 {
     for (;;) {
-        if (q.sp == 0) {
+        if (q.sp == stack.base) {
             return false;
         }
-        --q.sp;
-        const unsigned ref = stack[q.sp * stride];
+        q.sp -= TraceStack<unsigned>::kStride;
+        const unsigned ref = loadEntry(stack, q.sp);
         if (ref == kExitMarker) {
             q.changeSpace(q.origin, q.dir);
             q.inst_pos = kNoPrim;
@@ -672,19 +717,19 @@ enum TraceLoop : int { kLoopNodesThenLeaf = 0, kLoopOneStep = 1, kLoopQuery = 2 
 template <bool COUNT, bool HOLD, typename Stack>
 static __device__ __noinline__ bool traceSceneOutOfLine(const DevScene& s, float3 origin, float3 dir, float tmin,
                                                         float& tmax, const SkipRule& skip, TraceHit& hit,
-                                                        Stack* stack, int stride, int stack_size,
-                                                        unsigned int* error_flag, TraversalCounts* counts, bool any);
+                                                        Stack stack, unsigned int* error_flag,
+                                                        TraversalCounts* counts, bool any);
 
 template <int LOOP, typename Stack>
-__device__ __forceinline__ bool traceAdvance(const DevScene& s, TraceState& q, const SkipRule& skip, Stack* stack,
-                                             int stride, int stack_size, unsigned int* error_flag,
-                                             TraversalCounts* counts, bool any)
+__device__ __forceinline__ bool traceAdvance(const DevScene& s, TraceState& q, const SkipRule& skip,
+                                             const Stack& stack, unsigned int* error_flag, TraversalCounts* counts,
+                                             bool any)
 {
     if constexpr (LOOP == kLoopQuery) {
         float tmax = q.tmax;
         TraceHit hit;
-        q.found = traceSceneOutOfLine<false, false>(s, q.origin, q.dir, q.tmin, tmax, skip, hit, stack, stride,
-                                                    stack_size, error_flag, nullptr, any);
+        q.found = traceSceneOutOfLine<false, false>(s, q.origin, q.dir, q.tmin, tmax, skip, hit, stack,
+                                                    error_flag, nullptr, any);
         if (q.found) {
             q.tmax = tmax;
             q.hit = hit;
@@ -694,20 +739,20 @@ __device__ __forceinline__ bool traceAdvance(const DevScene& s, TraceState& q, c
     q.settle();
     int step = kStepDescend;
     if constexpr (LOOP == kLoopOneStep) {
-        step = (q.ref & kLeafBit) == 0u ? nodeStep(s.nodes, q, stack, stride, stack_size, error_flag, counts)
-                                        : leafStep(s, q, skip, stack, stride, stack_size, error_flag, counts, any);
+        step = (q.ref & kLeafBit) == 0u ? nodeStep(s.nodes, q, stack, error_flag, counts)
+                                        : leafStep(s, q, skip, stack, error_flag, counts, any);
     } else {
         while (step == kStepDescend && (q.ref & kLeafBit) == 0u) {
-            step = nodeStep(s.nodes, q, stack, stride, stack_size, error_flag, counts);
+            step = nodeStep(s.nodes, q, stack, error_flag, counts);
         }
         if (step == kStepDescend) {
-            step = leafStep(s, q, skip, stack, stride, stack_size, error_flag, counts, any);
+            step = leafStep(s, q, skip, stack, error_flag, counts, any);
         }
     }
     if (step == kStepFinished) {
         return false;
     }
-    return step == kStepDescend || popNext(q, stack, stride);
+    return step == kStepDescend || popNext(q, stack);
 }
 
 // Traverses the scene for the nearest hit in (tmin, tmax) (any = false), or for
@@ -726,15 +771,14 @@ __device__ __forceinline__ bool traceAdvance(const DevScene& s, TraceState& q, c
 // wavefront's persistent kernels, whose 96-register budget then spills.
 template <bool HOLD, typename Stack>
 __device__ __forceinline__ bool traceSceneBody(const DevScene& s, float3 origin, float3 dir, float tmin, float& tmax,
-                                               const SkipRule& skip, TraceHit& hit, Stack* stack, int stride,
-                                               int stack_size, unsigned int* error_flag, TraversalCounts* counts,
-                                               bool any)
+                                               const SkipRule& skip, TraceHit& hit, const Stack& stack,
+                                               unsigned int* error_flag, TraversalCounts* counts, bool any)
 {
     if (counts != nullptr) {
         counts->rays += 1;
     }
     TraceState q;
-    if (!traceBegin(s, q, origin, dir, tmin, tmax)) {
+    if (!traceBegin(s, q, stack.base, origin, dir, tmin, tmax)) {
         return false;
     }
     if (counts != nullptr) {
@@ -744,9 +788,9 @@ __device__ __forceinline__ bool traceSceneBody(const DevScene& s, float3 origin,
     for (;;) {
         q.settle();
         const int step = (q.ref & kLeafBit) == 0u
-                             ? nodeStep(HOLD ? held_nodes : s.nodes, q, stack, stride, stack_size, error_flag, counts)
-                             : leafStep(s, q, skip, stack, stride, stack_size, error_flag, counts, any);
-        if (step == kStepFinished || (step == kStepPop && !popNext(q, stack, stride))) {
+                             ? nodeStep(HOLD ? held_nodes : s.nodes, q, stack, error_flag, counts)
+                             : leafStep(s, q, skip, stack, error_flag, counts, any);
+        if (step == kStepFinished || (step == kStepPop && !popNext(q, stack))) {
             break;
         }
     }
@@ -764,11 +808,11 @@ __device__ __forceinline__ bool traceSceneBody(const DevScene& s, float3 origin,
 template <bool COUNT, bool HOLD, typename Stack>
 static __device__ __noinline__ bool traceSceneOutOfLine(const DevScene& s, float3 origin, float3 dir, float tmin,
                                                         float& tmax, const SkipRule& skip, TraceHit& hit,
-                                                        Stack* stack, int stride, int stack_size,
-                                                        unsigned int* error_flag, TraversalCounts* counts, bool any)
+                                                        Stack stack, unsigned int* error_flag,
+                                                        TraversalCounts* counts, bool any)
 {
-    return traceSceneBody<HOLD>(s, origin, dir, tmin, tmax, skip, hit, stack, stride, stack_size, error_flag,
-                                COUNT ? counts : nullptr, any);
+    return traceSceneBody<HOLD>(s, origin, dir, tmin, tmax, skip, hit, stack, error_flag, COUNT ? counts : nullptr,
+                                any);
 }
 
 // A query from a caller that keeps its state across the call (the megakernel),
@@ -779,25 +823,24 @@ static __device__ __noinline__ bool traceSceneOutOfLine(const DevScene& s, float
 // without it `counts` is ignored.
 template <bool INLINE = false, bool COUNT = false, typename Stack>
 ALB_DEV bool traceQuery(const DevScene& s, float3 origin, float3 dir, float tmin, float& tmax, const SkipRule& skip,
-                        TraceHit& hit, Stack* stack, int stride, int stack_size, unsigned int* error_flag,
-                        TraversalCounts* counts, bool any)
+                        TraceHit& hit, const Stack& stack, unsigned int* error_flag, TraversalCounts* counts,
+                        bool any)
 {
     if constexpr (INLINE) {
-        return traceSceneBody<true>(s, origin, dir, tmin, tmax, skip, hit, stack, stride, stack_size, error_flag,
+        return traceSceneBody<true>(s, origin, dir, tmin, tmax, skip, hit, stack, error_flag,
                                     COUNT ? counts : nullptr, any);
     } else {
-        return traceSceneOutOfLine<COUNT, true>(s, origin, dir, tmin, tmax, skip, hit, stack, stride, stack_size,
-                                                error_flag, counts, any);
+        return traceSceneOutOfLine<COUNT, true>(s, origin, dir, tmin, tmax, skip, hit, stack, error_flag, counts,
+                                                any);
     }
 }
 
 template <bool ANY, bool INLINE = false, bool COUNT = false, typename Stack>
 ALB_DEV bool traceScene(const DevScene& s, float3 origin, float3 dir, float tmin, float& tmax, const SkipRule& skip,
-                        TraceHit& hit, Stack* stack, int stride, int stack_size, unsigned int* error_flag,
+                        TraceHit& hit, const Stack& stack, unsigned int* error_flag,
                         TraversalCounts* counts = nullptr)
 {
-    return traceQuery<INLINE, COUNT>(s, origin, dir, tmin, tmax, skip, hit, stack, stride, stack_size, error_flag,
-                                     counts, ANY);
+    return traceQuery<INLINE, COUNT>(s, origin, dir, tmin, tmax, skip, hit, stack, error_flag, counts, ANY);
 }
 
 } // namespace albedo_b200

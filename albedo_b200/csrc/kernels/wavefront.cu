@@ -316,8 +316,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) extendKernel(const WfJ
     const int ended = kQRegen0 + (parity ^ 1);
     const int count = ctl->count[in];
     const WfSlots& sl = b.slots;
-    unsigned* const lane_stack = ref_stack + threadIdx.x;
-    const int stride = static_cast<int>(blockDim.x);
+    const auto lane_stack = TraceStack<unsigned>::of(ref_stack + threadIdx.x, STACK);
     WarpFetch fetch{0, 0, fetch_batch, false};
     TraceState q;
     SkipRule skip = SkipRule::none();
@@ -334,13 +333,13 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) extendKernel(const WfJ
             const float4 d = sl.ray_d[s];
             const uint4 k = sl.skip[s];
             skip = {k.x, k.y, static_cast<int>(k.z), kNoPrim};
-            active = traceBegin(*scene, q, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), 0.0f, INFINITY);
+            active = traceBegin(*scene, q, lane_stack.base, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), 0.0f, INFINITY);
             finished = !active;
         }
         if (__ballot_sync(0xFFFFFFFFu, active || finished) == 0u) {
             break;
         }
-        if (active && !traceAdvance<LOOP>(*scene, q, skip, lane_stack, stride, STACK, error_flag, nullptr, false)) {
+        if (active && !traceAdvance<LOOP>(*scene, q, skip, lane_stack, error_flag, nullptr, false)) {
             active = false;
             finished = true;
         }
@@ -469,8 +468,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) shadowKernel(const WfJ
     const int count = ctl->count[kQShadow];
     const int* const order = binned ? b.binned : b.queue[kQShadow];
     const WfSlots& sl = b.slots;
-    unsigned* const lane_stack = ref_stack + threadIdx.x;
-    const int stride = static_cast<int>(blockDim.x);
+    const auto lane_stack = TraceStack<unsigned>::of(ref_stack + threadIdx.x, STACK);
     WarpFetch fetch{0, 0, fetch_batch, false};
     TraceState q;
     SkipRule skip = SkipRule::none();
@@ -487,13 +485,13 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) shadowKernel(const WfJ
             const float4 d = sl.shadow_d[s];
             const uint4 k = sl.shadow_skip[s];
             skip = {k.x, k.y, static_cast<int>(k.z), __float_as_uint(d.w)};
-            active = traceBegin(*scene, q, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), 0.0f, o.w);
+            active = traceBegin(*scene, q, lane_stack.base, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), 0.0f, o.w);
             finished = !active;
         }
         if (__ballot_sync(0xFFFFFFFFu, active || finished) == 0u) {
             break;
         }
-        if (active && !traceAdvance<LOOP>(*scene, q, skip, lane_stack, stride, STACK, error_flag, nullptr, true)) {
+        if (active && !traceAdvance<LOOP>(*scene, q, skip, lane_stack, error_flag, nullptr, true)) {
             active = false;
             finished = true;
         }
@@ -603,10 +601,10 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) traceModesKernel(const
                                                                          unsigned int* out_tri)
 {
     extern __shared__ uint2 stack[];
-    uint2* const lane_stack = stack + threadIdx.x;
-    // The persistent modes use the 4-byte stack entries of the wavefront's kernels.
-    unsigned* const lane_refs = reinterpret_cast<unsigned*>(stack) + threadIdx.x;
-    const int stride = static_cast<int>(blockDim.x);
+    // Mode 0 uses 8-byte stack entries, the persistent modes the 4-byte entries of
+    // the wavefront's kernels.
+    const auto lane_stack = TraceStack<uint2>::of(stack + threadIdx.x, STACK);
+    const auto lane_refs = TraceStack<unsigned>::of(reinterpret_cast<unsigned*>(stack) + threadIdx.x, STACK);
     const auto store = [&](int i, bool found, const TraceHit& hit) {
         out_hit[i] = found ? 1 : 0;
         out_t[i] = found ? __float_as_uint(hit.t) : 0u;
@@ -620,8 +618,8 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) traceModesKernel(const
             float tmax = t_max;
             const float3 o = mk(rays[6 * i], rays[6 * i + 1], rays[6 * i + 2]);
             const float3 d = mk(rays[6 * i + 3], rays[6 * i + 4], rays[6 * i + 5]);
-            const bool found = traceQuery(scene, o, d, t_min, tmax, SkipRule::none(), hit, lane_stack, stride, STACK,
-                                          error_flag, nullptr, any);
+            const bool found = traceQuery(scene, o, d, t_min, tmax, SkipRule::none(), hit, lane_stack, error_flag,
+                                          nullptr, any);
             store(i, found, hit);
         }
         return;
@@ -637,7 +635,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) traceModesKernel(const
             i = next;
             const float3 o = mk(rays[6 * i], rays[6 * i + 1], rays[6 * i + 2]);
             const float3 d = mk(rays[6 * i + 3], rays[6 * i + 4], rays[6 * i + 5]);
-            active = traceBegin(scene, q, o, d, t_min, t_max);
+            active = traceBegin(scene, q, lane_refs.base, o, d, t_min, t_max);
             finished = !active;
         }
         if (__ballot_sync(0xFFFFFFFFu, active || finished) == 0u) {
@@ -646,14 +644,13 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) traceModesKernel(const
         bool more = false;
         if (active) {
             if (mode == 3) {
-                more = traceAdvance<kLoopQuery>(scene, q, SkipRule::none(), lane_refs, stride, STACK, error_flag,
-                                                nullptr, any);
+                more = traceAdvance<kLoopQuery>(scene, q, SkipRule::none(), lane_refs, error_flag, nullptr, any);
             } else if (mode == 2) {
-                more = traceAdvance<kLoopOneStep>(scene, q, SkipRule::none(), lane_refs, stride, STACK, error_flag,
-                                                  nullptr, any);
+                more = traceAdvance<kLoopOneStep>(scene, q, SkipRule::none(), lane_refs, error_flag, nullptr,
+                                                  any);
             } else {
-                more = traceAdvance<kLoopNodesThenLeaf>(scene, q, SkipRule::none(), lane_refs, stride, STACK,
-                                                        error_flag, nullptr, any);
+                more = traceAdvance<kLoopNodesThenLeaf>(scene, q, SkipRule::none(), lane_refs, error_flag,
+                                                        nullptr, any);
             }
         }
         if (active && !more) {
