@@ -82,13 +82,18 @@ struct TravRay {
     std::uint32_t planes; // bit a set when inv[a] is negative (-0 directions included): the box test's near planes
     bool usable;          // |d|^2 is a normal number
 
-    ALB_DEV void setup(float3 origin, float3 dir)
+    // `triangles`: the space holds triangles, whose test needs the shear
+    // (kx .. sz); without any, world space takes the box and sphere parts alone.
+    ALB_DEV void setup(float3 origin, float3 dir, bool triangles)
     {
         o = origin;
         inv = mk(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z);
         neg = (dir.x < 0.0f ? 1u : 0u) | (dir.y < 0.0f ? 2u : 0u) | (dir.z < 0.0f ? 4u : 0u);
         planes = (signbit(inv.x) ? 1u : 0u) | (signbit(inv.y) ? 2u : 0u) | (signbit(inv.z) ? 4u : 0u);
         usable = isNormalF(lengthSquared(dir));
+        if (!triangles) {
+            return;
+        }
         const float mx = fabsf(dir.x);
         const float my = fabsf(dir.y);
         const float mz = fabsf(dir.z);
@@ -103,7 +108,7 @@ struct TravRay {
         }
         sx = comp(dir, kx) / dz;
         sy = comp(dir, ky) / dz;
-        sz = 1.0f / dz;
+        sz = comp(inv, kz); // 1 / dz
     }
 };
 
@@ -207,6 +212,29 @@ ALB_DEV T rdot(T ax, T ay, T az, T bx, T by, T bz)
     return radd(radd(rmul(ax, bx), rmul(ay, by)), rmul(az, bz));
 }
 
+// Whether a sphere seen from outside (c > 0) has no root in (tmin, tmax),
+// decided without the test's divisions and square root; false leaves it to them.
+// - Moving away (h > 0): q = -(h + sqrt(disc)) is negative, so both roots, q / a
+//   and c / q, are negative or zero and fail tmin < t for tmin >= 0.
+// - Approaching: both roots are at least c / q, where q = -h + sqrt(disc) and
+//   disc = h^2 - a c < h^2 in exact arithmetic. The test's disc = a (r^2 - l^2)
+//   is off by less than 32 u a |oc|^2 (u: half an ulp of 1; |l| and r are at
+//   most |oc|), which is under 3200 u h^2 when h^2 >= a |oc|^2 / 100, so q <
+//   2.001 |h| and no root is below c / (2.001 |h|). The factor 2.01 covers the
+//   products' own rounding.
+// Inside a room of 1e4-radius walls most tests end here: half the walls are
+// behind the ray and most others beyond its hit. With the shear set up only
+// where triangles are tested, 298.8 -> 278.9 ms for the instanced trefoils
+// (960x540, 64 samples) and 8.48 -> 8.35 ms for the sphere room (320x180, 16).
+template <typename T>
+ALB_DEV bool beyondRange(T a, T h, T c, T oc2, T tmin, T tmax)
+{
+    if (h > T(0)) {
+        return tmin >= T(0);
+    }
+    return rmul(h, h) >= rmul(T(0.01), rmul(a, oc2)) && c > rmul(rmul(T(-2.01), h), tmax);
+}
+
 // Haines' sphere test in precision T (geometry/sphere.cpp:92-135), returning the
 // nearest root strictly inside (tmin, tmax), honouring the skip mode.
 template <typename T>
@@ -219,7 +247,11 @@ ALB_DEV bool sphereRoot(T ox, T oy, T oz, T dx, T dy, T dz, T cx, T cy, T cz, T 
     const T a = rdot(dx, dy, dz, dx, dy, dz);
     const T h = rdot(dx, dy, dz, ocx, ocy, ocz);
     const T r2 = rmul(radius, radius);
-    const T c = rsub(rdot(ocx, ocy, ocz, ocx, ocy, ocz), r2);
+    const T oc2 = rdot(ocx, ocy, ocz, ocx, ocy, ocz);
+    const T c = rsub(oc2, r2);
+    if (c > T(0) && beyondRange(a, h, c, oc2, tmin, tmax)) {
+        return false;
+    }
     const T k = h / a;
     const T lx = rsub(ocx, rmul(dx, k));
     const T ly = rsub(ocy, rmul(dy, k));
@@ -382,10 +414,10 @@ struct TraceState {
         r.inv = d;
         resetup = true;
     }
-    ALB_DEV void settle()
+    ALB_DEV void settle(const DevScene& s)
     {
         if (resetup) {
-            r.setup(r.o, r.inv);
+            r.setup(r.o, r.inv, inst_pos != kNoPrim || s.world_triangles != 0u);
             resetup = false;
         }
     }
@@ -414,7 +446,7 @@ ALB_DEV bool traceBegin(const DevScene& s, TraceState& q, unsigned stack_base, f
     if (s.tlas_root == kEmptyChild) {
         return false;
     }
-    q.r.setup(origin, dir);
+    q.changeSpace(origin, dir);
     return true;
 }
 
@@ -736,7 +768,7 @@ __device__ __forceinline__ bool traceAdvance(const DevScene& s, TraceState& q, c
         }
         return false;
     }
-    q.settle();
+    q.settle(s);
     int step = kStepDescend;
     if constexpr (LOOP == kLoopOneStep) {
         step = (q.ref & kLeafBit) == 0u ? nodeStep(s.nodes, q, stack, error_flag, counts)
@@ -786,7 +818,7 @@ __device__ __forceinline__ bool traceSceneBody(const DevScene& s, float3 origin,
     }
     const DevNode* const held_nodes = s.nodes;
     for (;;) {
-        q.settle();
+        q.settle(s);
         const int step = (q.ref & kLeafBit) == 0u
                              ? nodeStep(HOLD ? held_nodes : s.nodes, q, stack, error_flag, counts)
                              : leafStep(s, q, skip, stack, error_flag, counts, any);
