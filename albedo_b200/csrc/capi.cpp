@@ -278,6 +278,7 @@ struct albedo_scene {
         dev.light_count = static_cast<std::uint32_t>(image.lights.size());
         dev.sky_light = image.sky_light;
         dev.object_count = static_cast<std::uint32_t>(image.objects.size());
+        dev.triangle_count = static_cast<std::uint32_t>(image.triangles.size());
         dev.world_triangles = host.triangles.empty() ? 0u : 1u;
         error_flag = DeviceBuffer{sizeof(unsigned int)};
         check(cudaMemset(error_flag.ptr, 0, sizeof(unsigned int)), "cudaMemset");

@@ -161,6 +161,7 @@ struct DevScene {
     std::uint32_t light_count;
     std::int32_t sky_light;            // light index of the sky, or -1
     std::uint32_t object_count;
+    std::uint32_t triangle_count;
     std::uint32_t world_triangles;     // 1 when triangles are objects of their own (in world space)
 };
 

@@ -33,6 +33,8 @@ struct RenderArgs {
     // per SM the kernel is compiled for: 3 or 4). 0 picks the default (16, 3).
     int tile_width;
     int blocks_per_sm;
+    // Lanes of each warp that take a pixel (1, 2, 4, ..., 32); the launcher sets it.
+    int warp_pixels;
     // Nonzero: the traversal is inlined into the kernel (3 blocks per SM, path
     // estimator) instead of called out of line.
     int inline_traversal;

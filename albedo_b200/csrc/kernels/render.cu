@@ -25,6 +25,19 @@ constexpr int kTileW = 16; // default tile: 16 x 8 pixels
 #endif
 constexpr int kMegaBlocksPerSm = ALBEDO_MEGA_BLOCKS_PER_SM;
 
+// Pixels a block renders: warp_pixels in each of its four warps.
+__host__ __device__ inline int blockPixels(const RenderArgs& args) { return kBlock / 32 * args.warp_pixels; }
+
+// Width of a block's tile: the shape's for full warps, near-square for fewer
+// pixels (8 x 8, 8 x 4, 4 x 4, 4 x 2, 2 x 2).
+__host__ __device__ inline int tileWidth(const RenderArgs& args)
+{
+    if (args.warp_pixels == 32) {
+        return args.tile_width > 0 ? args.tile_width : kTileW;
+    }
+    return args.warp_pixels >= 8 ? 8 : (args.warp_pixels >= 2 ? 4 : 2);
+}
+
 // Per-pixel running sums: FP64, or FP32 with Kahan compensation.
 template <int ACC>
 struct PixelSums;
@@ -102,19 +115,25 @@ __global__ void __launch_bounds__(kBlock, MINB) megakernel(const DevScene scene,
     const TraceContext<INL != 0, COUNT, INL == 1, Entry> ctx{TraceStack<Entry>::of(stack + threadIdx.x, STACK),
                                                              error_flag, COUNT ? &counts : nullptr};
     int x, y, slot;
+    const int lanes = args.warp_pixels;
+    const int lane = static_cast<int>(threadIdx.x) & 31;
+    if (lane >= lanes) {
+        return;
+    }
+    const int place = (static_cast<int>(threadIdx.x) >> 5) * lanes + lane;
     if (args.pixels != nullptr) {
-        slot = blockIdx.x * kBlock + threadIdx.x;
+        slot = blockIdx.x * blockPixels(args) + place;
         if (slot >= args.pixel_count) {
             return;
         }
         x = args.pixels[slot].x;
         y = args.pixels[slot].y;
     } else {
-        const int tile_w = args.tile_width > 0 ? args.tile_width : kTileW;
-        const int tile_h = kBlock / tile_w;
+        const int tile_w = tileWidth(args);
+        const int tile_h = blockPixels(args) / tile_w;
         const int tiles_x = (args.width + tile_w - 1) / tile_w;
-        x = (blockIdx.x % tiles_x) * tile_w + static_cast<int>(threadIdx.x) % tile_w;
-        y = (blockIdx.x / tiles_x) * tile_h + static_cast<int>(threadIdx.x) / tile_w;
+        x = (blockIdx.x % tiles_x) * tile_w + place % tile_w;
+        y = (blockIdx.x / tiles_x) * tile_h + place / tile_w;
         if (x >= args.width || y >= args.height) {
             return;
         }
@@ -277,11 +296,49 @@ constexpr int kCountEntry = static_cast<int>(sizeof(StackEntry<true>));
 int megaBlocks(const RenderArgs& args)
 {
     if (args.pixels != nullptr) {
-        return (args.pixel_count + kBlock - 1) / kBlock;
+        return (args.pixel_count + blockPixels(args) - 1) / blockPixels(args);
     }
-    const int tile_w = args.tile_width > 0 ? args.tile_width : kTileW;
-    const int tile_h = kBlock / tile_w;
+    const int tile_w = tileWidth(args);
+    const int tile_h = blockPixels(args) / tile_w;
     return ((args.width + tile_w - 1) / tile_w) * ((args.height + tile_h - 1) / tile_h);
+}
+
+// How many lanes of a warp take a pixel (RenderArgs::warp_pixels): 32, or fewer
+// for an image too small to fill the GPU with full warps. A pixel's samples run
+// in sequence on its lane, so a small image takes as long as its slowest warps,
+// and a warp of divergent lanes takes several times as long as one lane alone:
+// spreading the pixels over the idle warp slots shortens each warp's chain. The
+// smallest power of two is taken whose warps are at most 12 per SM, the resident
+// warps of the default shape (3 blocks of 4), or 3 per SM for scenes of spheres
+// with hardly any triangle, whose short queries leave less divergence to save
+// and whose FP64 sphere tests cost a warp the same for one lane as for 32.
+//
+// Measured, 9 samples, depth 10, full warps -> this rule, in ms (trefoils of
+// 12,288 triangles / 20,480-triangle icosphere / soup of 30,000):
+//   64x36 4.04 / 3.60 / 5.72 -> 1.79 / 1.65 / 1.87
+//   96x54 4.18 / 4.28 / 7.21 -> 2.44 / 2.26 / 3.08
+//   128x72 4.16 / 4.68 / 7.83 -> 3.03 / 3.17 / 4.41
+//   192x108 4.54 / 5.00 / 8.37 -> 4.56 / 4.35 / 6.36
+// From 256x144 on full warps win for some of them (trefoils 5.48, and 6.21 at
+// 16 pixels a warp). Sphere room: 32x18 1.54 -> 0.66, 64x36 1.79 -> 1.26, 96x54
+// 1.86 -> 1.60; at 128x72 full warps, 1.87, beat 16 pixels a warp, 1.95.
+cudaError_t chooseWarpPixels(const DevScene& scene, RenderArgs& args)
+{
+    int device = 0;
+    int sms = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) {
+        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    }
+    constexpr std::uint32_t kFewTriangles = 256;
+    const long long warps = static_cast<long long>(sms) * (scene.triangle_count < kFewTriangles ? 3 : 12);
+    const long long pixels =
+        args.pixels != nullptr ? args.pixel_count : static_cast<long long>(args.width) * args.height;
+    args.warp_pixels = 1;
+    while (args.warp_pixels < 32 && pixels > warps * args.warp_pixels) {
+        args.warp_pixels *= 2;
+    }
+    return e;
 }
 
 // Launches `kernel` over `blocks` blocks with a STACK-entry shared-memory stack
@@ -302,10 +359,12 @@ cudaError_t launchStacked(Kernel kernel, int blocks, cudaStream_t stream, Args..
 
 } // namespace
 
-cudaError_t launchMegakernelCounting(const DevScene& scene, const DevCamera& camera, const RenderArgs& args,
+cudaError_t launchMegakernelCounting(const DevScene& scene, const DevCamera& camera, const RenderArgs& render,
                                      PixelAccum* accum, unsigned int* error_flag, int stack_capacity,
                                      unsigned long long* totals, cudaStream_t stream)
 {
+    RenderArgs args = render;
+    args.warp_pixels = 32;
     return withStack(stack_capacity, [&](auto size) {
         constexpr int S = decltype(size)::value;
         return launchStacked<S, kCountEntry>(megakernel<S, kEstimatorPath, true>, megaBlocks(args), stream, scene, camera, args,
@@ -355,9 +414,14 @@ cudaError_t launchPathMegakernel(const DevScene& scene, const DevCamera& camera,
                             args, accum, error_flag, no_totals);
 }
 
-cudaError_t launchMegakernel(const DevScene& scene, const DevCamera& camera, const RenderArgs& args, PixelAccum* accum,
-                             unsigned int* error_flag, int stack_capacity, cudaStream_t stream)
+cudaError_t launchMegakernel(const DevScene& scene, const DevCamera& camera, const RenderArgs& render,
+                             PixelAccum* accum, unsigned int* error_flag, int stack_capacity, cudaStream_t stream)
 {
+    RenderArgs args = render;
+    const cudaError_t chosen = chooseWarpPixels(scene, args);
+    if (chosen != cudaSuccess) {
+        return chosen;
+    }
     return withStack(stack_capacity, [&](auto size) {
         constexpr int S = decltype(size)::value;
         unsigned long long* no_totals = nullptr;
