@@ -738,8 +738,9 @@ __device__ __forceinline__ bool popNext(TraceState& q, const TraceStack<unsigned
 //   kLoopNodesThenLeaf  descend through interior nodes, then handle the leaf
 //                       reached, so the lanes of a warp move through each phase
 //                       together;
-//   kLoopOneStep        one node or one leaf, so lanes return to take new rays
-//                       sooner;
+//   kLoopOneStep        one node or one leaf, so lanes whose query ended take
+//                       new rays soon (the wavefront's kernels do so once
+//                       enough of a warp's lanes have ended);
 //   kLoopQuery          the whole query in one turn, through the out-of-line
 //                       traversal (a function of its own: the calling kernel's
 //                       state is saved around the call, and the traversal loop

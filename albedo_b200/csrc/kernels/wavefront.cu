@@ -299,6 +299,40 @@ __global__ void __launch_bounds__(128) binScatterKernel(WfBuffers b)
     }
 }
 
+// One turn of a persistent warp's queries: true for a lane whose query ended.
+// All 32 lanes call it together; `active` lanes have a query in flight.
+//
+// With one step a turn (kLoopOneStep) the warp stays here until fewer than
+// kRefillLanes queries are left, so that the lanes that ended file their results
+// and take new rays together: filing costs a few hundred instructions and two
+// dependent memory accesses whatever the number of lanes, and most single steps
+// end the query of only one or two. Once the queue is empty the warp finishes
+// what it holds.
+// Measured against the whole query a turn (fetches of 32 rays), ms: instanced
+// trefoils 960x540 at 16 samples 58.2 -> 54.4, 81,920-triangle icosphere 36.5 ->
+// 34.2, 200,003-triangle soup 853x481 80.2 -> 72.2, 16-job batch 124.5 -> 120.7;
+// filing after every step 60.4 / 38.3 / 79.3 / 137.2. Thresholds of 8 to 24 lanes
+// are within 1% of 16, and fetches of 16 rays beat 32 by 2-5% and 64 by far.
+constexpr int kRefillLanes = 16;
+
+template <int LOOP>
+ALB_DEV bool traceWarp(const DevScene* scene, TraceState& q, const SkipRule& skip, const TraceStack<unsigned>& stack,
+                       unsigned int* error_flag, bool any, bool drained, bool& active)
+{
+    bool ended = false;
+    unsigned busy = 0u;
+    do {
+        if (active && !traceAdvance<LOOP>(*scene, q, skip, stack, error_flag, nullptr, any)) {
+            active = false;
+            ended = true;
+        }
+        if constexpr (LOOP == kLoopOneStep) {
+            busy = __ballot_sync(0xFFFFFFFFu, active);
+        }
+    } while (LOOP == kLoopOneStep && busy != 0u && (drained || __popc(busy) >= kRefillLanes));
+    return ended;
+}
+
 // Closest hit of every ray in the extend queue. The kernel is persistent: a lane
 // whose query ends files the result and takes the next queued ray, so a warp is
 // not held by its slowest ray. Each query runs the same traversal steps, in the
@@ -339,10 +373,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) extendKernel(const WfJ
         if (__ballot_sync(0xFFFFFFFFu, active || finished) == 0u) {
             break;
         }
-        if (active && !traceAdvance<LOOP>(*scene, q, skip, lane_stack, error_flag, nullptr, false)) {
-            active = false;
-            finished = true;
-        }
+        finished |= traceWarp<LOOP>(scene, q, skip, lane_stack, error_flag, false, fetch.drained, active);
         if (finished) {
             int cls = -1;
             if (q.found) {
@@ -491,10 +522,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) shadowKernel(const WfJ
         if (__ballot_sync(0xFFFFFFFFu, active || finished) == 0u) {
             break;
         }
-        if (active && !traceAdvance<LOOP>(*scene, q, skip, lane_stack, error_flag, nullptr, true)) {
-            active = false;
-            finished = true;
-        }
+        finished |= traceWarp<LOOP>(scene, q, skip, lane_stack, error_flag, true, fetch.drained, active);
         if (finished && !q.found) {
             const float4 c = sl.shadow_c[s];
             float4 r = sl.result[s];
