@@ -27,14 +27,12 @@ constexpr std::size_t kMaxDevices = 64;
 
 constexpr std::size_t alignUp(std::size_t n) { return (n + 255) & ~static_cast<std::size_t>(255); }
 
-constexpr std::size_t kF4 = alignUp(sizeof(float4) * kNoAllocMaxSlots);
-constexpr std::size_t kF2 = alignUp(sizeof(float2) * kNoAllocMaxSlots);
-constexpr std::size_t kU2 = alignUp(sizeof(ulonglong2) * kNoAllocMaxSlots);
+constexpr std::size_t kRecords = alignUp(kWfSlotRecord * kNoAllocMaxSlots);
 constexpr std::size_t kQueue = alignUp(sizeof(int) * kNoAllocMaxSlots);
 constexpr std::size_t kControl = alignUp(sizeof(WfControl));
 constexpr std::size_t kJob = alignUp(sizeof(WfJob));
 constexpr std::size_t kJobDone = alignUp(sizeof(unsigned long long));
-constexpr std::size_t kScratchBytes = 12 * kF4 + kF2 + kU2 + kQueueCount * kQueue + kControl + kJob + kJobDone;
+constexpr std::size_t kScratchBytes = kWfSlotRecords * kRecords + kQueueCount * kQueue + kControl + kJob + kJobDone;
 
 // The scratch. In host code this name is a host-side stand-in, not a device
 // address; the host passes the address cudaGetSymbolAddress returns.
@@ -79,21 +77,7 @@ WfBuffers carve(void* base, int slots, WfJob** job)
         return r;
     };
     WfBuffers b{};
-    WfSlots& s = b.slots;
-    s.ray_o = static_cast<float4*>(take(kF4));
-    s.ray_d = static_cast<float4*>(take(kF4));
-    s.throughput = static_cast<float4*>(take(kF4));
-    s.result = static_cast<float4*>(take(kF4));
-    s.arrival = static_cast<float4*>(take(kF4));
-    s.skip = static_cast<uint4*>(take(kF4));
-    s.where = static_cast<int4*>(take(kF4));
-    s.hit = static_cast<float4*>(take(kF4));
-    s.shadow_o = static_cast<float4*>(take(kF4));
-    s.shadow_d = static_cast<float4*>(take(kF4));
-    s.shadow_skip = static_cast<uint4*>(take(kF4));
-    s.shadow_c = static_cast<float4*>(take(kF4));
-    s.hit_b = static_cast<float2*>(take(kF2));
-    s.rng = static_cast<ulonglong2*>(take(kU2));
+    placeSlots(b.slots, kRecords, take);
     for (int q = 0; q < kQueueCount; ++q) {
         b.queue[q] = static_cast<int*>(take(kQueue));
     }

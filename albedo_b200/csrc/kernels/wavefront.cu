@@ -84,24 +84,25 @@ ALB_DEV int findJob(const WfJob* jobs, int job_count, long long item)
     return lo;
 }
 
-ALB_DEV void storeRay(const WfSlots& sl, int s, const PathState& p)
+ALB_DEV void storeRay(const WfSlots& sl, int s, int job, const PathState& p)
 {
-    sl.ray_o[s] = make_float4(p.o.x, p.o.y, p.o.z, p.arrival_pdf);
-    sl.ray_d[s] = make_float4(p.d.x, p.d.y, p.d.z, p.arrival_specular ? 1.0f : 0.0f);
-    sl.throughput[s] = make_float4(p.throughput.x, p.throughput.y, p.throughput.z, 0.0f);
-    sl.result[s] = make_float4(p.result.x, p.result.y, p.result.z, 0.0f);
-    sl.arrival[s] = make_float4(p.arrival_origin.x, p.arrival_origin.y, p.arrival_origin.z, 0.0f);
-    sl.skip[s] = make_uint4(p.skip.object_pos, p.skip.tri_pos, static_cast<unsigned>(p.skip.sphere_mode), 0u);
+    sl.ray[s].o = make_float4(p.o.x, p.o.y, p.o.z, p.arrival_pdf);
+    sl.ray[s].d = make_float4(p.d.x, p.d.y, p.d.z, p.arrival_specular ? 1.0f : 0.0f);
+    sl.path[s].throughput = make_float4(p.throughput.x, p.throughput.y, p.throughput.z, 0.0f);
+    sl.path[s].result = make_float4(p.result.x, p.result.y, p.result.z, 0.0f);
+    sl.from[s].arrival = make_float4(p.arrival_origin.x, p.arrival_origin.y, p.arrival_origin.z, 0.0f);
+    sl.from[s].skip = make_uint4(p.skip.object_pos, p.skip.tri_pos, static_cast<unsigned>(p.skip.sphere_mode),
+                                 static_cast<unsigned>(job));
 }
 
 ALB_DEV void loadPath(const WfSlots& sl, int s, int depth, PathState& p)
 {
-    const float4 o = sl.ray_o[s];
-    const float4 d = sl.ray_d[s];
-    const float4 t = sl.throughput[s];
-    const float4 r = sl.result[s];
-    const float4 a = sl.arrival[s];
-    const uint4 k = sl.skip[s];
+    const float4 o = sl.ray[s].o;
+    const float4 d = sl.ray[s].d;
+    const float4 t = sl.path[s].throughput;
+    const float4 r = sl.path[s].result;
+    const float4 a = sl.from[s].arrival;
+    const uint4 k = sl.from[s].skip;
     p.o = mk(o.x, o.y, o.z);
     p.arrival_pdf = o.w;
     p.d = mk(d.x, d.y, d.z);
@@ -147,13 +148,13 @@ __global__ void __launch_bounds__(128) regenKernel(const WfJob* __restrict__ job
     const int stride = static_cast<int>(gridDim.x * blockDim.x);
     for (int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x); i < count; i += stride) {
         const int s = b.queue[in][i];
-        int4 w = sl.where[s];
+        int4 w = sl.state[s].where;
         bool start = false;
         int done_job = -1; // the job whose pixel this slot finished
         Pcg32 g;
         if (w.x >= 0) {
             const WfJob& job = jobs[w.x];
-            const float4 r = sl.result[s];
+            const float4 r = sl.path[s].result;
             PixelAccum& acc = job.accum[w.y];
             acc.r += r.x;
             acc.g += r.y;
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(128) regenKernel(const WfJob* __restrict__ job
             w.z += 1;
             if (w.z < job.samples_per_axis * job.samples_per_axis) {
                 start = true;
-                const ulonglong2 st = sl.rng[s];
+                const ulonglong2 st = sl.state[s].rng;
                 g = {st.x, st.y};
             } else {
                 done_job = w.x;
@@ -186,11 +187,11 @@ __global__ void __launch_bounds__(128) regenKernel(const WfJob* __restrict__ job
             PathState p;
             startSample(job.camera, p, g, w.y % job.width, w.y / job.width, w.z, n, 1.0f / static_cast<float>(n),
                         static_cast<float>(job.width), static_cast<float>(job.height));
-            storeRay(sl, s, p);
-            sl.rng[s] = make_ulonglong2(g.state, g.inc);
+            storeRay(sl, s, w.x, p);
+            sl.state[s].rng = make_ulonglong2(g.state, g.inc);
             w.w = 0;
         }
-        sl.where[s] = w;
+        sl.state[s].where = w;
         pushSlot(b.queue[out], &ctl->count[out], s, start);
         pushSlot(b.queue[kQParked], &ctl->count[kQParked], s, !start);
     }
@@ -253,9 +254,9 @@ __global__ void __launch_bounds__(128) binKeysKernel(const WfJob* __restrict__ j
     const int stride = static_cast<int>(gridDim.x * blockDim.x);
     for (int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x); i < count; i += stride) {
         const int s = b.queue[in][i];
-        const int job = b.slots.where[s].x;
-        const float4 o = SHADOW ? b.slots.shadow_o[s] : b.slots.ray_o[s];
-        const float4 d = SHADOW ? b.slots.shadow_d[s] : b.slots.ray_d[s];
+        const int job = b.slots.state[s].where.x;
+        const float4 o = SHADOW ? b.slots.query[s].a : b.slots.ray[s].o;
+        const float4 d = SHADOW ? b.slots.query[s].b : b.slots.ray[s].d;
         const unsigned int key = rayBinKey(jobs[job], job, o, d);
         b.bin_key[i] = key;
         static_cast<void>(groupedAdd(b.bin_count, key));
@@ -384,10 +385,10 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) extendKernel(const WfJ
         bool finished = false;
         if (i >= 0) {
             s = order[i];
-            scene = &jobs[sl.where[s].x].scene;
-            const float4 o = sl.ray_o[s];
-            const float4 d = sl.ray_d[s];
-            const uint4 k = sl.skip[s];
+            const float4 o = sl.ray[s].o;
+            const float4 d = sl.ray[s].d;
+            const uint4 k = sl.from[s].skip;
+            scene = &jobs[k.w].scene;
             skip = {k.x, k.y, static_cast<int>(k.z), kNoPrim};
             active = traceBegin(*scene, q, lane_stack.base, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), 0.0f, INFINITY);
             finished = !active;
@@ -399,24 +400,24 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) extendKernel(const WfJ
         if (finished) {
             int cls = -1;
             if (q.found) {
-                sl.hit[s] = make_float4(q.hit.t, __uint_as_float(q.hit.obj_pos), __uint_as_float(q.hit.tri_pos),
+                sl.query[s].a = make_float4(q.hit.t, __uint_as_float(q.hit.obj_pos), __uint_as_float(q.hit.tri_pos),
                                         q.hit.b0);
-                sl.hit_b[s] = make_float2(q.hit.b1, q.hit.b2);
+                sl.query[s].b = make_float4(q.hit.b1, q.hit.b2, 0.0f, 0.0f);
                 cls = materialClass(*scene, q.hit.obj_pos);
             } else {
-                const float4 o = sl.ray_o[s];
-                const float4 d = sl.ray_d[s];
+                const float4 o = sl.ray[s].o;
+                const float4 d = sl.ray[s].d;
                 PathState p;
                 p.d = mk(d.x, d.y, d.z);
                 p.arrival_pdf = o.w;
                 p.arrival_specular = d.w != 0.0f;
-                const float4 t = sl.throughput[s];
+                const float4 t = sl.path[s].throughput;
                 const float3 e = weightedSky(*scene, p);
-                float4 r = sl.result[s];
+                float4 r = sl.path[s].result;
                 r.x += t.x * e.x;
                 r.y += t.y * e.y;
                 r.z += t.z * e.z;
-                sl.result[s] = r;
+                sl.path[s].result = r;
             }
             pushSlot(b.queue[ended], &ctl->count[ended], s, !q.found);
             pushSlot(b.queue[kQDiffuse], &ctl->count[kQDiffuse], s, cls == kClassDiffuse);
@@ -440,15 +441,15 @@ __global__ void __launch_bounds__(128) shadeKernel(const WfJob* __restrict__ job
     const int stride = static_cast<int>(gridDim.x * blockDim.x);
     for (int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x); i < count; i += stride) {
         const int s = b.queue[in][i];
-        int4 w = sl.where[s];
+        int4 w = sl.state[s].where;
         const WfJob& job = jobs[w.x];
         const DevScene& scene = job.scene;
         PathState p;
         loadPath(sl, s, w.w, p);
-        const float4 h = sl.hit[s];
-        const float2 hb = sl.hit_b[s];
+        const float4 h = sl.query[s].a;
+        const float4 hb = sl.query[s].b;
         const TraceHit hit{h.x, __float_as_uint(h.y), __float_as_uint(h.z), h.w, hb.x, hb.y};
-        const ulonglong2 st = sl.rng[s];
+        const ulonglong2 st = sl.state[s].rng;
         Pcg32 g{st.x, st.y};
         Surface sf;
         resolveHit(scene, p.o, p.d, hit, sf);
@@ -463,11 +464,12 @@ __global__ void __launch_bounds__(128) shadeKernel(const WfJob* __restrict__ job
                 const float3 c = p.throughput * nc.contribution;
                 if (nc.needs_test) {
                     shadow = true;
-                    sl.shadow_o[s] = make_float4(nc.origin.x, nc.origin.y, nc.origin.z, nc.range_max);
-                    sl.shadow_d[s] = make_float4(nc.dir.x, nc.dir.y, nc.dir.z, __uint_as_float(nc.skip.light_object_pos));
-                    sl.shadow_skip[s] = make_uint4(nc.skip.object_pos, nc.skip.tri_pos,
-                                                   static_cast<unsigned>(nc.skip.sphere_mode), 0u);
-                    sl.shadow_c[s] = make_float4(c.x, c.y, c.z, 0.0f);
+                    sl.query[s].a = make_float4(nc.origin.x, nc.origin.y, nc.origin.z, nc.range_max);
+                    sl.query[s].b = make_float4(nc.dir.x, nc.dir.y, nc.dir.z, __uint_as_float(nc.skip.light_object_pos));
+                    sl.pending[s].skip = make_uint4(nc.skip.object_pos, nc.skip.tri_pos,
+                                                   static_cast<unsigned>(nc.skip.sphere_mode),
+                                                        static_cast<unsigned>(w.x));
+                    sl.pending[s].c = make_float4(c.x, c.y, c.z, 0.0f);
                 } else {
                     p.result = p.result + c;
                 }
@@ -500,9 +502,9 @@ __global__ void __launch_bounds__(128) shadeKernel(const WfJob* __restrict__ job
                 }
             }
         }
-        storeRay(sl, s, p);
-        sl.rng[s] = make_ulonglong2(g.state, g.inc);
-        sl.where[s] = w;
+        storeRay(sl, s, w.x, p);
+        sl.state[s].rng = make_ulonglong2(g.state, g.inc);
+        sl.state[s].where = w;
         pushSlot(b.queue[kQShadow], &ctl->count[kQShadow], s, shadow);
         pushSlot(b.queue[next], &ctl->count[next], s, alive);
         pushSlot(b.queue[ended], &ctl->count[ended], s, !alive);
@@ -533,10 +535,10 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) shadowKernel(const WfJ
         bool finished = false;
         if (i >= 0) {
             s = order[i];
-            scene = &jobs[sl.where[s].x].scene;
-            const float4 o = sl.shadow_o[s];
-            const float4 d = sl.shadow_d[s];
-            const uint4 k = sl.shadow_skip[s];
+            const float4 o = sl.query[s].a;
+            const float4 d = sl.query[s].b;
+            const uint4 k = sl.pending[s].skip;
+            scene = &jobs[k.w].scene;
             skip = {k.x, k.y, static_cast<int>(k.z), __float_as_uint(d.w)};
             active = traceBegin(*scene, q, lane_stack.base, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), 0.0f, o.w);
             finished = !active;
@@ -546,12 +548,12 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) shadowKernel(const WfJ
         }
         finished |= traceWarp<LOOP>(scene, q, skip, lane_stack, error_flag, true, fetch.drained, active);
         if (finished && !q.found) {
-            const float4 c = sl.shadow_c[s];
-            float4 r = sl.result[s];
+            const float4 c = sl.pending[s].c;
+            float4 r = sl.path[s].result;
             r.x += c.x;
             r.y += c.y;
             r.z += c.z;
-            sl.result[s] = r;
+            sl.path[s].result = r;
         }
     }
 }
@@ -578,7 +580,7 @@ __global__ void resetKernel(WfBuffers b, unsigned long long total_items, int job
 {
     const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
     if (i < b.slot_count) {
-        b.slots.where[i] = make_int4(-1, 0, 0, 0);
+        b.slots.state[i].where = make_int4(-1, 0, 0, 0);
         b.queue[kQRegen0][i] = i;
     }
     if (i < job_count) {

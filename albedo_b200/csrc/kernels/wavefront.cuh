@@ -4,6 +4,7 @@
 
 #include "launch.hpp"
 
+#include <cstddef>
 #include <cstdint>
 
 namespace albedo_b200 {
@@ -31,25 +32,63 @@ struct WfJob {
 constexpr int kBinBits = 14;
 constexpr int kBinCount = 1 << kBinBits;
 
-// Path slots, one record per field group so a gather of one slot reads whole
-// 16-byte records. A slot owns one pixel for all of that pixel's samples, so its
-// PCG32 stream advances exactly as the reference's per-pixel generator does.
-struct WfSlots {
-    float4* ray_o;      // origin xyz, arrival pdf
-    float4* ray_d;      // direction xyz, arrival-specular flag (0 or 1)
-    float4* throughput; // xyz, unused
-    float4* result;     // radiance gathered so far xyz, unused
-    float4* arrival;    // previous scattering point xyz, unused
-    uint4* skip;        // object position, triangle position, sphere mode, unused
-    ulonglong2* rng;    // PCG32 state, increment
-    int4* where;        // job (-1: idle), pixel index in the job, sample index, depth
-    float4* hit;        // t, object position bits, triangle position bits, b0
-    float2* hit_b;      // b1, b2
-    float4* shadow_o;   // shadow ray origin xyz, range end
-    float4* shadow_d;   // shadow ray direction xyz, area-light object position bits
-    uint4* shadow_skip; // object position, triangle position, sphere mode, unused
-    float4* shadow_c;   // contribution if unoccluded xyz, unused
+// Path slots, in records of 32 bytes: what one kernel reads or writes of a slot
+// together. A queue lists slots in any order, so every record is a gather of its
+// own, and L2 and DRAM move whole 32-byte sectors: 16-byte records in arrays of
+// their own moved each sector for half its bytes. A slot owns one pixel for all
+// of that pixel's samples, so its PCG32 stream advances exactly as the
+// reference's per-pixel generator does.
+struct alignas(32) WfRay {
+    float4 o; // origin xyz, arrival pdf
+    float4 d; // direction xyz, arrival-specular flag (0 or 1)
 };
+struct alignas(32) WfPath {
+    float4 throughput; // xyz, unused
+    float4 result;     // radiance gathered so far xyz, unused
+};
+struct alignas(32) WfFrom {
+    float4 arrival; // previous scattering point xyz, unused
+    uint4 skip;     // object position, triangle position, sphere mode, job
+};
+struct alignas(32) WfState {
+    ulonglong2 rng; // PCG32 state, increment
+    int4 where;     // job (-1: idle), pixel index in the job, sample index, depth
+};
+// From the extend kernel to the shade kernel the hit, from the shade kernel to
+// the shadow kernel the shadow ray (a slot's hit is read before its shadow ray
+// is written, by the same thread).
+struct alignas(32) WfQuery {
+    float4 a; // hit: t, object position bits, triangle position bits, b0; shadow ray: origin xyz, range end
+    float4 b; // hit: b1, b2, unused; shadow ray: direction xyz, area-light object position bits
+};
+struct alignas(32) WfPending {
+    uint4 skip; // object position, triangle position, sphere mode, job
+    float4 c;   // contribution if unoccluded xyz, unused
+};
+
+struct WfSlots {
+    WfRay* ray;
+    WfPath* path;
+    WfFrom* from;
+    WfState* state;
+    WfQuery* query;
+    WfPending* pending;
+};
+constexpr std::size_t kWfSlotRecord = 32;
+constexpr int kWfSlotRecords = 6;
+
+// Points the six record arrays at memory that take(bytes) hands out,
+// `array_bytes` each.
+template <typename Take>
+void placeSlots(WfSlots& slots, std::size_t array_bytes, Take&& take)
+{
+    slots.ray = static_cast<WfRay*>(take(array_bytes));
+    slots.path = static_cast<WfPath*>(take(array_bytes));
+    slots.from = static_cast<WfFrom*>(take(array_bytes));
+    slots.state = static_cast<WfState*>(take(array_bytes));
+    slots.query = static_cast<WfQuery*>(take(array_bytes));
+    slots.pending = static_cast<WfPending*>(take(array_bytes));
+}
 
 enum WfQueueId : int {
     kQExtend0 = 0,

@@ -33,13 +33,11 @@ WavefrontEngine::WavefrontEngine(int slot_count, int job_capacity)
         throw std::invalid_argument{"the wavefront engine needs at least one slot and one job"};
     }
     const auto n{static_cast<std::size_t>(slot_count)};
-    const std::size_t f4{align256(n * sizeof(float4))};
-    const std::size_t f2{align256(n * sizeof(float2))};
-    const std::size_t u2{align256(n * sizeof(ulonglong2))};
+    const std::size_t records{align256(n * kWfSlotRecord)};
     const std::size_t q{align256(n * sizeof(int))};
     const auto jobs{static_cast<std::size_t>(job_capacity)};
     const std::size_t bins{align256(kBinCount * sizeof(unsigned int))};
-    const std::size_t total{12 * f4 + f2 + u2 + kQueueCount * q + align256(sizeof(WfControl)) +
+    const std::size_t total{kWfSlotRecords * records + kQueueCount * q + align256(sizeof(WfControl)) +
                             align256(jobs * sizeof(unsigned long long)) + align256(jobs * sizeof(WfJob)) + 2 * q +
                             2 * bins};
     cudaCheck(cudaMalloc(&slab_, total), "wavefront slots");
@@ -50,21 +48,7 @@ WavefrontEngine::WavefrontEngine(int slot_count, int job_capacity)
         p += bytes;
         return r;
     };
-    WfSlots& s{buffers_.slots};
-    s.ray_o = static_cast<float4*>(take(f4));
-    s.ray_d = static_cast<float4*>(take(f4));
-    s.throughput = static_cast<float4*>(take(f4));
-    s.result = static_cast<float4*>(take(f4));
-    s.arrival = static_cast<float4*>(take(f4));
-    s.skip = static_cast<uint4*>(take(f4));
-    s.where = static_cast<int4*>(take(f4));
-    s.hit = static_cast<float4*>(take(f4));
-    s.shadow_o = static_cast<float4*>(take(f4));
-    s.shadow_d = static_cast<float4*>(take(f4));
-    s.shadow_skip = static_cast<uint4*>(take(f4));
-    s.shadow_c = static_cast<float4*>(take(f4));
-    s.hit_b = static_cast<float2*>(take(f2));
-    s.rng = static_cast<ulonglong2*>(take(u2));
+    placeSlots(buffers_.slots, records, take);
     for (int i{0}; i < kQueueCount; ++i) {
         buffers_.queue[i] = static_cast<int*>(take(q));
     }

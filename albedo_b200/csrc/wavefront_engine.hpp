@@ -27,7 +27,7 @@ struct WfShape {
 
 class WavefrontEngine {
 public:
-    // `slot_count` path slots (264 bytes each, queues and ray binning included)
+    // `slot_count` path slots (240 bytes each, queues and ray binning included)
     // and a table of `job_capacity`
     // jobs on the current device.
     WavefrontEngine(int slot_count, int job_capacity);
