@@ -8,6 +8,7 @@
 #include "host/scene_file.hpp"
 #include "host/srgb.hpp"
 #include "kernels/launch.hpp"
+#include "query_pool.hpp"
 #include "wavefront_engine.hpp"
 
 #include <algorithm>
@@ -205,6 +206,34 @@ BasicMaterialDesc basicFrom(const albedo_basic_material& m)
 
 } // namespace
 
+namespace {
+
+// A committed scene's share in its device's ray-query buffers (runQueries).
+class QueryShare {
+public:
+    QueryShare() = default;
+    QueryShare(const QueryShare&) = delete;
+    QueryShare& operator=(const QueryShare&) = delete;
+    ~QueryShare()
+    {
+        if (device_ >= 0) {
+            releaseQueryBuffers(device_);
+        }
+    }
+    void hold(int device)
+    {
+        if (device_ < 0) {
+            retainQueryBuffers(device);
+            device_ = device;
+        }
+    }
+
+private:
+    int device_{-1};
+};
+
+} // namespace
+
 struct albedo_scene {
     HostScene host;
     bool prepared{false};
@@ -214,6 +243,7 @@ struct albedo_scene {
     int stack_capacity{0};
     std::vector<DeviceBuffer> buffers;
     DeviceBuffer error_flag;
+    QueryShare query_share;
     // Ray-binning cells of the scene (coherenceGrid), for the wavefront.
     std::array<float, 4> grid{};
     // Megakernel launch shape the autotuner kept for this scene (0: default).
@@ -282,6 +312,9 @@ struct albedo_scene {
         dev.world_triangles = host.triangles.empty() ? 0u : 1u;
         error_flag = DeviceBuffer{sizeof(unsigned int)};
         check(cudaMemset(error_flag.ptr, 0, sizeof(unsigned int)), "cudaMemset");
+        int device{0};
+        check(cudaGetDevice(&device), "cudaGetDevice");
+        query_share.hold(device);
         committed = true;
     }
 
@@ -1619,39 +1652,49 @@ int albedo_scene_check(const albedo_scene* scene)
     });
 }
 
+namespace {
+
+// runQueries with its CUDA failures as device errors.
+void hostQueries(int64_t count, std::span<const QueryInput> inputs, std::span<const QueryOutput> outputs,
+                 const QueryLaunch& launch)
+{
+    try {
+        runQueries(count, inputs, outputs, launch);
+    } catch (const std::bad_alloc&) {
+        throw;
+    } catch (const std::exception& e) {
+        throw DeviceError{e.what()};
+    }
+}
+
+} // namespace
+
 int albedo_trace_host(const albedo_scene* scene, const float* rays, int64_t count, float t_min, float t_max,
                       int32_t* hit, float* t, int32_t* object, int32_t* triangle, float* point, float* normal,
                       float* shading_normal, int32_t* front)
 {
     return guarded([&] {
         scene->requireCommitted();
-        const auto n{static_cast<std::size_t>(count)};
-        DeviceBuffer d_rays{uploadRaw(rays, 6 * n)};
-        DeviceBuffer d_hit{n * sizeof(int)};
-        DeviceBuffer d_t{n * sizeof(float)};
-        DeviceBuffer d_object{n * sizeof(int)};
-        DeviceBuffer d_triangle{n * sizeof(int)};
         const bool geometry{point != nullptr};
-        DeviceBuffer d_point{geometry ? 3 * n * sizeof(float) : 0};
-        DeviceBuffer d_normal{geometry ? 3 * n * sizeof(float) : 0};
-        DeviceBuffer d_shading{geometry ? 3 * n * sizeof(float) : 0};
-        DeviceBuffer d_front{geometry ? n * sizeof(int) : 0};
-        TraceOutputs out{d_hit.as<int>(),   d_t.as<float>(),      d_object.as<int>(),   d_triangle.as<int>(),
-                         d_point.as<float>(), d_normal.as<float>(), d_shading.as<float>(), d_front.as<int>()};
-        check(launchTrace(scene->dev, d_rays.as<float>(), static_cast<int>(count), t_min, t_max, out,
-                          scene->error_flag.as<unsigned int>(), scene->stack_capacity, nullptr),
-              "trace launch");
-        check(cudaDeviceSynchronize(), "trace");
-        download(hit, d_hit, n);
-        download(t, d_t, n);
-        download(object, d_object, n);
-        download(triangle, d_triangle, n);
-        if (geometry) {
-            download(point, d_point, 3 * n);
-            download(normal, d_normal, 3 * n);
-            download(shading_normal, d_shading, 3 * n);
-            download(front, d_front, n);
-        }
+        const std::size_t three{geometry ? 3 * sizeof(float) : 0};
+        const QueryInput inputs[]{{rays, 6 * sizeof(float)}};
+        const QueryOutput outputs[]{{hit, sizeof(int)},       {t, sizeof(float)}, {object, sizeof(int)},
+                                    {triangle, sizeof(int)},  {point, three},     {normal, three},
+                                    {shading_normal, three},  {front, geometry ? sizeof(int) : 0}};
+        hostQueries(count, inputs, outputs, [&](void* const* in, void* const* out, int n, cudaStream_t stream) {
+            const auto floats = [&](int i) { return static_cast<float*>(out[i]); };
+            const auto ints = [&](int i) { return static_cast<int*>(out[i]); };
+            const TraceOutputs to{ints(0),
+                                  floats(1),
+                                  ints(2),
+                                  ints(3),
+                                  geometry ? floats(4) : nullptr,
+                                  geometry ? floats(5) : nullptr,
+                                  geometry ? floats(6) : nullptr,
+                                  geometry ? ints(7) : nullptr};
+            return launchTrace(scene->dev, static_cast<const float*>(in[0]), n, t_min, t_max, to,
+                               scene->error_flag.as<unsigned int>(), scene->stack_capacity, stream);
+        });
         scene->collectKernelError();
     });
 }
@@ -1661,15 +1704,13 @@ int albedo_occluded_host(const albedo_scene* scene, const float* rays, const flo
 {
     return guarded([&] {
         scene->requireCommitted();
-        const auto n{static_cast<std::size_t>(count)};
-        DeviceBuffer d_rays{uploadRaw(rays, 6 * n)};
-        DeviceBuffer d_tmax{uploadRaw(t_max, n)};
-        DeviceBuffer d_out{n * sizeof(int)};
-        check(launchOccluded(scene->dev, d_rays.as<float>(), d_tmax.as<float>(), static_cast<int>(count),
-                             d_out.as<int>(), scene->error_flag.as<unsigned int>(), scene->stack_capacity, nullptr),
-              "occluded launch");
-        check(cudaDeviceSynchronize(), "occluded");
-        download(occluded, d_out, n);
+        const QueryInput inputs[]{{rays, 6 * sizeof(float)}, {t_max, sizeof(float)}};
+        const QueryOutput outputs[]{{occluded, sizeof(int)}};
+        hostQueries(count, inputs, outputs, [&](void* const* in, void* const* out, int n, cudaStream_t stream) {
+            return launchOccluded(scene->dev, static_cast<const float*>(in[0]), static_cast<const float*>(in[1]), n,
+                                  static_cast<int*>(out[0]), scene->error_flag.as<unsigned int>(),
+                                  scene->stack_capacity, stream);
+        });
         scene->collectKernelError();
     });
 }

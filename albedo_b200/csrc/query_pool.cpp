@@ -1,0 +1,287 @@
+// Worker buffers of host-array ray queries, and the chunk loop.
+#include "query_pool.hpp"
+
+#include <algorithm>
+#include <array>
+#include <atomic>
+#include <condition_variable>
+#include <cstring>
+#include <exception>
+#include <format>
+#include <map>
+#include <memory>
+#include <mutex>
+#include <new>
+#include <stdexcept>
+#include <thread>
+#include <vector>
+
+namespace albedo_b200 {
+
+namespace {
+
+// Rays of a chunk: a call is split into kMaxWorkers chunks, of no fewer rays
+// than make a full wave of threads worth launching and no more than a worker's
+// buffers hold (2.8 MB pinned and as much device memory, 22 MB of each per
+// device at most).
+constexpr std::int64_t kMinChunk{16384};
+constexpr std::int64_t kMaxChunk{32768};
+constexpr std::size_t kMaxWorkers{8};
+constexpr std::size_t kArrayAlign{256};
+constexpr std::size_t kSlotBytes{kMaxChunk * kMaxQueryRayBytes + 2 * kMaxQueryArrays * kArrayAlign};
+
+void cudaCheck(cudaError_t e, const char* what)
+{
+    if (e == cudaErrorMemoryAllocation) {
+        throw std::bad_alloc{};
+    }
+    if (e != cudaSuccess) {
+        throw std::runtime_error{std::format("{}: {}", what, cudaGetErrorString(e))};
+    }
+}
+
+// One worker's stream, pinned buffer and device buffer.
+struct Slot {
+    cudaStream_t stream{nullptr};
+    char* pinned{nullptr};
+    char* device{nullptr};
+
+    Slot() = default;
+    Slot(const Slot&) = delete;
+    Slot& operator=(const Slot&) = delete;
+    void allocate()
+    {
+        cudaCheck(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "query stream");
+        void* p{nullptr};
+        cudaCheck(cudaMallocHost(&p, kSlotBytes), "query staging");
+        pinned = static_cast<char*>(p);
+        cudaCheck(cudaMalloc(&p, kSlotBytes), "query buffers");
+        device = static_cast<char*>(p);
+    }
+    ~Slot()
+    {
+        if (device != nullptr) {
+            cudaFree(device);
+        }
+        if (pinned != nullptr) {
+            cudaFreeHost(pinned);
+        }
+        if (stream != nullptr) {
+            cudaStreamDestroy(stream);
+        }
+    }
+};
+
+// A device's slots: at most kMaxWorkers, made as they are needed; a worker that
+// finds all of them in use waits for one.
+struct DevicePool {
+    std::mutex mutex;
+    std::condition_variable freed;
+    std::vector<std::unique_ptr<Slot>> idle;
+    std::size_t made{0};
+    int scenes{0};
+
+    std::unique_ptr<Slot> take()
+    {
+        std::unique_lock lock{mutex};
+        freed.wait(lock, [&] { return !idle.empty() || made < kMaxWorkers; });
+        if (!idle.empty()) {
+            std::unique_ptr<Slot> slot{std::move(idle.back())};
+            idle.pop_back();
+            return slot;
+        }
+        ++made;
+        lock.unlock();
+        auto slot{std::make_unique<Slot>()};
+        try {
+            slot->allocate();
+        } catch (...) {
+            slot.reset();
+            drop();
+            throw;
+        }
+        return slot;
+    }
+    // Puts a slot back; with no scene left on the device it is given up.
+    void give(std::unique_ptr<Slot> slot)
+    {
+        {
+            const std::lock_guard lock{mutex};
+            if (scenes > 0) {
+                idle.push_back(std::move(slot));
+                freed.notify_one();
+                return;
+            }
+        }
+        slot.reset();
+        drop();
+    }
+    void drop()
+    {
+        const std::lock_guard lock{mutex};
+        --made;
+        freed.notify_one();
+    }
+};
+
+DevicePool& poolOf(int device)
+{
+    static std::mutex table_mutex;
+    // Never destroyed: freeing device memory from a static destructor at exit
+    // would run after the CUDA runtime has shut down.
+    static auto* table{new std::map<int, std::unique_ptr<DevicePool>>};
+    const std::lock_guard lock{table_mutex};
+    std::unique_ptr<DevicePool>& entry{(*table)[device]};
+    if (!entry) {
+        entry = std::make_unique<DevicePool>();
+    }
+    return *entry;
+}
+
+// A slot held by a worker.
+class HeldSlot {
+public:
+    explicit HeldSlot(DevicePool& pool) : pool_{pool}, slot_{pool.take()} {}
+    // A worker that failed may leave copies in flight that use the buffers.
+    ~HeldSlot()
+    {
+        cudaStreamSynchronize(slot_->stream);
+        pool_.give(std::move(slot_));
+    }
+    HeldSlot(const HeldSlot&) = delete;
+    HeldSlot& operator=(const HeldSlot&) = delete;
+    Slot& operator*() const { return *slot_; }
+
+private:
+    DevicePool& pool_;
+    std::unique_ptr<Slot> slot_;
+};
+
+std::size_t aligned(std::size_t n) { return (n + kArrayAlign - 1) & ~(kArrayAlign - 1); }
+
+// Queries [first, first + n) of the call through one slot: inputs lie at the
+// slot's start, outputs behind them, each array on its own 256-byte boundary.
+void runChunk(const Slot& slot, std::size_t first, std::size_t n, std::span<const QueryInput> inputs,
+              std::span<const QueryOutput> outputs, const QueryLaunch& launch)
+{
+    std::array<void*, kMaxQueryArrays> device_in{};
+    std::array<void*, kMaxQueryArrays> device_out{};
+    std::size_t at{0};
+    for (std::size_t i{0}; i < inputs.size(); ++i) {
+        const std::size_t bytes{n * inputs[i].ray_bytes};
+        std::memcpy(slot.pinned + at, static_cast<const char*>(inputs[i].host) + first * inputs[i].ray_bytes, bytes);
+        device_in[i] = slot.device + at;
+        at += aligned(bytes);
+    }
+    const std::size_t results{at};
+    cudaCheck(cudaMemcpyAsync(slot.device, slot.pinned, results, cudaMemcpyHostToDevice, slot.stream), "upload");
+    for (std::size_t i{0}; i < outputs.size(); ++i) {
+        device_out[i] = slot.device + at;
+        at += aligned(n * outputs[i].ray_bytes);
+    }
+    cudaCheck(launch(device_in.data(), device_out.data(), static_cast<int>(n), slot.stream), "query launch");
+    cudaCheck(cudaMemcpyAsync(slot.pinned + results, slot.device + results, at - results, cudaMemcpyDeviceToHost,
+                              slot.stream),
+              "download");
+    cudaCheck(cudaStreamSynchronize(slot.stream), "queries");
+    at = results;
+    for (const QueryOutput& out : outputs) {
+        const std::size_t bytes{n * out.ray_bytes};
+        if (out.host != nullptr) {
+            std::memcpy(static_cast<char*>(out.host) + first * out.ray_bytes, slot.pinned + at, bytes);
+        }
+        at += aligned(bytes);
+    }
+}
+
+} // namespace
+
+void runQueries(std::int64_t count, std::span<const QueryInput> inputs, std::span<const QueryOutput> outputs,
+                const QueryLaunch& launch)
+{
+    if (count < 0) {
+        throw std::bad_alloc{};
+    }
+    if (count == 0) {
+        return;
+    }
+    std::size_t ray_bytes{0};
+    for (const QueryInput& in : inputs) {
+        ray_bytes += in.ray_bytes;
+    }
+    for (const QueryOutput& out : outputs) {
+        ray_bytes += out.ray_bytes;
+    }
+    if (ray_bytes > kMaxQueryRayBytes || inputs.size() > kMaxQueryArrays || outputs.size() > kMaxQueryArrays) {
+        throw std::logic_error{"a query takes more bytes a ray than a worker's buffers hold"};
+    }
+    int device{0};
+    cudaCheck(cudaGetDevice(&device), "cudaGetDevice");
+    DevicePool& pool{poolOf(device)};
+    const std::int64_t share{(count + static_cast<std::int64_t>(kMaxWorkers) - 1) /
+                             static_cast<std::int64_t>(kMaxWorkers)};
+    const std::int64_t chunk{std::clamp(share, kMinChunk, kMaxChunk)};
+    const std::int64_t chunks{(count + chunk - 1) / chunk};
+    std::atomic<std::int64_t> next{0};
+    const auto work = [&] {
+        const HeldSlot slot{pool};
+        for (std::int64_t c{next++}; c < chunks; c = next++) {
+            const std::int64_t first{c * chunk};
+            runChunk(*slot, static_cast<std::size_t>(first), static_cast<std::size_t>(std::min(chunk, count - first)),
+                     inputs, outputs, launch);
+        }
+    };
+    const std::size_t cores{std::max<std::size_t>(1, std::thread::hardware_concurrency())};
+    const std::size_t workers{std::min({kMaxWorkers, cores, static_cast<std::size_t>(chunks)})};
+    std::vector<std::exception_ptr> failed(workers);
+    {
+        std::vector<std::jthread> threads;
+        const auto guardedWork = [&](std::size_t k) {
+            try {
+                cudaCheck(cudaSetDevice(device), "cudaSetDevice");
+                work();
+            } catch (...) {
+                failed[k] = std::current_exception();
+                next = chunks;
+            }
+        };
+        threads.reserve(workers - 1);
+        try {
+            for (std::size_t k{1}; k < workers; ++k) {
+                threads.emplace_back(guardedWork, k);
+            }
+        } catch (const std::system_error&) {
+            // Fewer threads than asked for: the ones that started share the chunks.
+        }
+        guardedWork(0);
+    }
+    for (const std::exception_ptr& e : failed) {
+        if (e) {
+            std::rethrow_exception(e);
+        }
+    }
+}
+
+void retainQueryBuffers(int device)
+{
+    DevicePool& pool{poolOf(device)};
+    const std::lock_guard lock{pool.mutex};
+    ++pool.scenes;
+}
+
+void releaseQueryBuffers(int device)
+{
+    DevicePool& pool{poolOf(device)};
+    std::vector<std::unique_ptr<Slot>> given;
+    {
+        const std::lock_guard lock{pool.mutex};
+        if (--pool.scenes > 0) {
+            return;
+        }
+        given.swap(pool.idle);
+        pool.made -= given.size();
+        pool.freed.notify_all();
+    }
+}
+
+} // namespace albedo_b200
