@@ -322,11 +322,23 @@ __global__ void __launch_bounds__(128) binScatterKernel(WfBuffers b)
     }
 }
 
+// How many lanes of each warp of a persistent traversal kernel take rays: all 32,
+// or no more than spread a short queue over every resident warp. An iteration
+// waits for its slowest warp, and 32 divergent rays in one warp take several
+// times as long as one; a batch ends with a long tail of such iterations.
+// Measured, ms: 16-job batch 108.8 -> 105.1, trefoil frame at 16 samples 51.2 ->
+// 49.4, two-job batch 9.8 -> 8.8; at least 8 lanes a warp: 108.8, 51.0, 9.8.
+ALB_DEV int raysPerWarp(int count)
+{
+    const int warps = static_cast<int>(gridDim.x * blockDim.x / 32u);
+    return min(32, max(1, (count + warps - 1) / warps));
+}
+
 // One turn of a persistent warp's queries: true for a lane whose query ended.
 // All 32 lanes call it together; `active` lanes have a query in flight.
 //
-// With one step a turn (kLoopOneStep) the warp stays here until fewer than
-// kRefillLanes queries are left, so that the lanes that ended file their results
+// With one step a turn (kLoopOneStep) the warp stays here until fewer than half
+// its `lanes` have a query left, so that the lanes that ended file their results
 // and take new rays together: filing costs a few hundred instructions and two
 // dependent memory accesses whatever the number of lanes, and most single steps
 // end the query of only one or two. Once the queue is empty the warp finishes
@@ -336,11 +348,9 @@ __global__ void __launch_bounds__(128) binScatterKernel(WfBuffers b)
 // 34.2, 200,003-triangle soup 853x481 80.2 -> 72.2, 16-job batch 124.5 -> 120.7;
 // filing after every step 60.4 / 38.3 / 79.3 / 137.2. Thresholds of 8 to 24 lanes
 // are within 1% of 16, and fetches of 16 rays beat 32 by 2-5% and 64 by far.
-constexpr int kRefillLanes = 16;
-
 template <int LOOP>
 ALB_DEV bool traceWarp(const DevScene* scene, TraceState& q, const SkipRule& skip, const TraceStack<unsigned>& stack,
-                       unsigned int* error_flag, bool any, bool drained, bool& active)
+                       unsigned int* error_flag, bool any, bool drained, int lanes, bool& active)
 {
     bool ended = false;
     unsigned busy = 0u;
@@ -352,7 +362,7 @@ ALB_DEV bool traceWarp(const DevScene* scene, TraceState& q, const SkipRule& ski
         if constexpr (LOOP == kLoopOneStep) {
             busy = __ballot_sync(0xFFFFFFFFu, active);
         }
-    } while (LOOP == kLoopOneStep && busy != 0u && (drained || __popc(busy) >= kRefillLanes));
+    } while (LOOP == kLoopOneStep && busy != 0u && (drained || 2 * __popc(busy) >= lanes));
     return ended;
 }
 
@@ -374,14 +384,16 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) extendKernel(const WfJ
     const int count = ctl->count[in];
     const WfSlots& sl = b.slots;
     const auto lane_stack = TraceStack<unsigned>::of(ref_stack + threadIdx.x, STACK);
-    WarpFetch fetch{0, 0, fetch_batch, false};
+    const int lanes = raysPerWarp(count);
+    WarpFetch fetch{0, 0, min(fetch_batch, lanes), false};
+    const bool takes = static_cast<int>(threadIdx.x & 31u) < lanes;
     TraceState q;
     SkipRule skip = SkipRule::none();
     const DevScene* scene = nullptr;
     int s = -1;
     bool active = false;
     for (;;) {
-        const int i = fetch.take(&ctl->fetch_extend, count, !active);
+        const int i = fetch.take(&ctl->fetch_extend, count, takes && !active);
         bool finished = false;
         if (i >= 0) {
             s = order[i];
@@ -396,7 +408,8 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) extendKernel(const WfJ
         if (__ballot_sync(0xFFFFFFFFu, active || finished) == 0u) {
             break;
         }
-        finished |= traceWarp<LOOP>(scene, q, skip, lane_stack, error_flag, false, fetch.drained, active);
+        finished |= traceWarp<LOOP>(scene, q, skip, lane_stack, error_flag, false, fetch.drained, lanes,
+                                    active);
         if (finished) {
             int cls = -1;
             if (q.found) {
@@ -524,14 +537,16 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) shadowKernel(const WfJ
     const int* const order = binned ? b.binned : b.queue[kQShadow];
     const WfSlots& sl = b.slots;
     const auto lane_stack = TraceStack<unsigned>::of(ref_stack + threadIdx.x, STACK);
-    WarpFetch fetch{0, 0, fetch_batch, false};
+    const int lanes = raysPerWarp(count);
+    WarpFetch fetch{0, 0, min(fetch_batch, lanes), false};
+    const bool takes = static_cast<int>(threadIdx.x & 31u) < lanes;
     TraceState q;
     SkipRule skip = SkipRule::none();
     const DevScene* scene = nullptr;
     int s = -1;
     bool active = false;
     for (;;) {
-        const int i = fetch.take(&ctl->fetch_shadow, count, !active);
+        const int i = fetch.take(&ctl->fetch_shadow, count, takes && !active);
         bool finished = false;
         if (i >= 0) {
             s = order[i];
@@ -546,7 +561,8 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) shadowKernel(const WfJ
         if (__ballot_sync(0xFFFFFFFFu, active || finished) == 0u) {
             break;
         }
-        finished |= traceWarp<LOOP>(scene, q, skip, lane_stack, error_flag, true, fetch.drained, active);
+        finished |= traceWarp<LOOP>(scene, q, skip, lane_stack, error_flag, true, fetch.drained, lanes,
+                                    active);
         if (finished && !q.found) {
             const float4 c = sl.pending[s].c;
             float4 r = sl.path[s].result;
