@@ -20,11 +20,13 @@ namespace albedo_b200 {
 // shadow queries' traversal (by default as INLINE), COUNT counts the work into
 // `counts` (traceScene). Stack entries are unsigned (the child reference alone)
 // or uint2 (reference and entry distance).
-template <bool INLINE, bool COUNT = false, bool INLINE_SHADOW = INLINE, typename Entry = unsigned>
+template <bool INLINE, bool COUNT = false, bool INLINE_SHADOW = INLINE, typename Entry = unsigned,
+          bool PACKED = false>
 struct TraceContext {
     static constexpr bool kInline = INLINE;
     static constexpr bool kInlineShadow = INLINE_SHADOW;
     static constexpr bool kCount = COUNT;
+    static constexpr bool kPacked = PACKED; // nodeStep's
     TraceStack<Entry> stack;
     unsigned int* error_flag;
     TraversalCounts* counts; // null except in the counting variants
@@ -34,16 +36,16 @@ template <typename Ctx>
 ALB_DEV bool closestHit(const DevScene& s, const Ctx& c, float3 o, float3 d, const SkipRule& skip, TraceHit& hit)
 {
     float tmax = INFINITY;
-    return traceScene<false, Ctx::kInline, Ctx::kCount>(s, o, d, 0.0f, tmax, skip, hit, c.stack,
-                                                        c.error_flag, c.counts);
+    return traceScene<false, Ctx::kInline, Ctx::kCount, Ctx::kPacked>(s, o, d, 0.0f, tmax, skip, hit, c.stack,
+                                                                      c.error_flag, c.counts);
 }
 
 template <typename Ctx>
 ALB_DEV bool occluded(const DevScene& s, const Ctx& c, float3 o, float3 d, float tmax, const SkipRule& skip)
 {
     TraceHit hit;
-    return traceScene<true, Ctx::kInlineShadow, Ctx::kCount>(s, o, d, 0.0f, tmax, skip, hit, c.stack,
-                                                             c.error_flag, c.counts);
+    return traceScene<true, Ctx::kInlineShadow, Ctx::kCount, Ctx::kPacked>(s, o, d, 0.0f, tmax, skip, hit, c.stack,
+                                                                           c.error_flag, c.counts);
 }
 
 // Next-event estimation from one uniformly chosen light, MIS-weighted, before

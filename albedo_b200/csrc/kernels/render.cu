@@ -112,8 +112,8 @@ __global__ void __launch_bounds__(kBlock, MINB) megakernel(const DevScene scene,
     extern __shared__ uint2 stack_memory[];
     Entry* const stack = reinterpret_cast<Entry*>(stack_memory);
     TraversalCounts counts{0, 0, 0, 0, 0, 0};
-    const TraceContext<INL != 0, COUNT, INL == 1, Entry> ctx{TraceStack<Entry>::of(stack + threadIdx.x, STACK),
-                                                             error_flag, COUNT ? &counts : nullptr};
+    const TraceContext<INL != 0, COUNT, INL == 1, Entry, EST == kEstimatorPath> ctx{
+        TraceStack<Entry>::of(stack + threadIdx.x, STACK), error_flag, COUNT ? &counts : nullptr};
     int x, y, slot;
     const int lanes = args.warp_pixels;
     const int lane = static_cast<int>(threadIdx.x) & 31;

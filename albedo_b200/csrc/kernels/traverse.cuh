@@ -156,6 +156,17 @@ __device__ __forceinline__ float min3f(float a, float b, float c)
     return d;
 }
 
+// The range of a box from its near and far plane distances on each axis.
+__device__ __forceinline__ bool slabRange(float tnx, float tfx, float tny, float tfy, float tnz, float tfz, float tmin,
+                                          float tmax, float& entry)
+{
+    const float lo = max3f(tnx, tny, fmaxf(tnz, tmin));
+    const float f = min3f(tfx, tfy, tfz);
+    const float hi = fminf(fmaxf(__fmul_rn(f, kBoxExitWidening), __fmul_rn(f, 2.0f - kBoxExitWidening)), tmax);
+    entry = lo;
+    return lo <= hi;
+}
+
 // slabTest without branches, given the box's near and far planes on each axis:
 // lo and hi where the inverse direction's sign bit is clear, hi and lo where it
 // is set (a -0 direction component gives a -infinite inverse, so it counts as
@@ -182,17 +193,47 @@ __device__ __forceinline__ float min3f(float a, float b, float c)
 __device__ __forceinline__ bool slabTestOrdered(float nx, float fx, float ny, float fy, float nz, float fz,
                                                 const TravRay& r, float tmin, float tmax, float& entry)
 {
-    const float tnx = __fmul_rn(__fsub_rn(nx, r.o.x), r.inv.x);
-    const float tfx = __fmul_rn(__fsub_rn(fx, r.o.x), r.inv.x);
-    const float tny = __fmul_rn(__fsub_rn(ny, r.o.y), r.inv.y);
-    const float tfy = __fmul_rn(__fsub_rn(fy, r.o.y), r.inv.y);
-    const float tnz = __fmul_rn(__fsub_rn(nz, r.o.z), r.inv.z);
-    const float tfz = __fmul_rn(__fsub_rn(fz, r.o.z), r.inv.z);
-    const float lo = max3f(tnx, tny, fmaxf(tnz, tmin));
-    const float f = min3f(tfx, tfy, tfz);
-    const float hi = fminf(fmaxf(__fmul_rn(f, kBoxExitWidening), __fmul_rn(f, 2.0f - kBoxExitWidening)), tmax);
-    entry = lo;
-    return lo <= hi;
+    return slabRange(__fmul_rn(__fsub_rn(nx, r.o.x), r.inv.x), __fmul_rn(__fsub_rn(fx, r.o.x), r.inv.x),
+                     __fmul_rn(__fsub_rn(ny, r.o.y), r.inv.y), __fmul_rn(__fsub_rn(fy, r.o.y), r.inv.y),
+                     __fmul_rn(__fsub_rn(nz, r.o.z), r.inv.z), __fmul_rn(__fsub_rn(fz, r.o.z), r.inv.z), tmin, tmax,
+                     entry);
+}
+
+// Two FP32 values in one 64-bit register pair, and sm_100's packed add and
+// multiply, each rounding both halves as the scalar operation does.
+struct FloatPair {
+    unsigned long long bits;
+
+    ALB_DEV static FloatPair of(float a, float b)
+    {
+        FloatPair p;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(p.bits) : "f"(a), "f"(b));
+        return p;
+    }
+    ALB_DEV void get(float& a, float& b) const { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(bits)); }
+};
+ALB_DEV FloatPair radd(FloatPair a, FloatPair b)
+{
+    FloatPair c;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(c.bits) : "l"(a.bits), "l"(b.bits));
+    return c;
+}
+ALB_DEV FloatPair rmul(FloatPair a, FloatPair b)
+{
+    FloatPair c;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(c.bits) : "l"(a.bits), "l"(b.bits));
+    return c;
+}
+
+// The distances to four children's planes on one axis, (plane - o) * inv.
+ALB_DEV float4 planeDistances(const float4& planes, float o, float inv)
+{
+    const FloatPair minus_o = FloatPair::of(-o, -o);
+    const FloatPair inv2 = FloatPair::of(inv, inv);
+    float4 t;
+    rmul(radd(FloatPair::of(planes.x, planes.y), minus_o), inv2).get(t.x, t.y);
+    rmul(radd(FloatPair::of(planes.z, planes.w), minus_o), inv2).get(t.z, t.w);
+    return t;
 }
 
 // Explicitly rounded arithmetic: every product and sum rounds on its own, as the
@@ -537,7 +578,15 @@ ALB_DEV unsigned loadEntry(const TraceStack<unsigned>&, unsigned at)
 // per-octant table, the hit children set bits p_c of `hits`, the lowest set bit
 // is the next child and a child's entry lies above the entries of the set bits
 // beyond its own.
-template <typename Stack>
+//
+// PACKED computes the plane distances two at a time: half the instructions of
+// that part, but each axis's origin and inverse take a register pair. The path
+// estimator's megakernel (168 registers a thread) gains, ms: trefoils 277.6 ->
+// 270.4, icosphere 181.7 -> 179.9, soup 49.2 -> 48.8, sphere room 8.42 -> 8.24.
+// The others lose and keep the scalar form: the scatter-only estimator (140
+// registers) 172.2 -> 174.4 in the room at 1174x843, the persistent kernels (96)
+// 51.0 -> 51.4 for the trefoils.
+template <bool PACKED, typename Stack>
 __device__ __forceinline__ int nodeStep(const DevNode* nodes, TraceState& q, const Stack& stack,
                                         unsigned int* error_flag, TraversalCounts* counts)
 {
@@ -563,10 +612,24 @@ __device__ __forceinline__ int nodeStep(const DevNode* nodes, TraceState& q, con
     const float4 nz = __ldg(np + 4u + sz);
     const float4 fz = __ldg(np + (5u - sz));
     float e0, e1, e2, e3;
-    const bool h0 = slabTestOrdered(nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, r, q.tmin, q.tmax, e0);
-    const bool h1 = slabTestOrdered(nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, r, q.tmin, q.tmax, e1);
-    const bool h2 = slabTestOrdered(nx.z, fx.z, ny.z, fy.z, nz.z, fz.z, r, q.tmin, q.tmax, e2);
-    const bool h3 = slabTestOrdered(nx.w, fx.w, ny.w, fy.w, nz.w, fz.w, r, q.tmin, q.tmax, e3);
+    bool h0, h1, h2, h3;
+    if constexpr (PACKED) {
+        const float4 tnx = planeDistances(nx, r.o.x, r.inv.x);
+        const float4 tfx = planeDistances(fx, r.o.x, r.inv.x);
+        const float4 tny = planeDistances(ny, r.o.y, r.inv.y);
+        const float4 tfy = planeDistances(fy, r.o.y, r.inv.y);
+        const float4 tnz = planeDistances(nz, r.o.z, r.inv.z);
+        const float4 tfz = planeDistances(fz, r.o.z, r.inv.z);
+        h0 = slabRange(tnx.x, tfx.x, tny.x, tfy.x, tnz.x, tfz.x, q.tmin, q.tmax, e0);
+        h1 = slabRange(tnx.y, tfx.y, tny.y, tfy.y, tnz.y, tfz.y, q.tmin, q.tmax, e1);
+        h2 = slabRange(tnx.z, tfx.z, tny.z, tfy.z, tnz.z, tfz.z, q.tmin, q.tmax, e2);
+        h3 = slabRange(tnx.w, tfx.w, tny.w, tfy.w, tnz.w, tfz.w, q.tmin, q.tmax, e3);
+    } else {
+        h0 = slabTestOrdered(nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, r, q.tmin, q.tmax, e0);
+        h1 = slabTestOrdered(nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, r, q.tmin, q.tmax, e1);
+        h2 = slabTestOrdered(nx.z, fx.z, ny.z, fy.z, nz.z, fz.z, r, q.tmin, q.tmax, e2);
+        h3 = slabTestOrdered(nx.w, fx.w, ny.w, fy.w, nz.w, fz.w, r, q.tmin, q.tmax, e3);
+    }
     // The octant's byte of the table; child c's place is its bits 2c, 2c + 1.
     // Absent children (zero boxes) are tested too; their places lie beyond
     // those of the children present and are masked off.
@@ -747,7 +810,7 @@ __device__ __forceinline__ bool popNext(TraceState& q, const TraceStack<unsigned
 //                       has the registers to itself).
 enum TraceLoop : int { kLoopNodesThenLeaf = 0, kLoopOneStep = 1, kLoopQuery = 2 };
 
-template <bool COUNT, bool HOLD, typename Stack>
+template <bool COUNT, bool HOLD, bool PACKED, typename Stack>
 static __device__ __noinline__ bool traceSceneOutOfLine(const DevScene& s, float3 origin, float3 dir, float tmin,
                                                         float& tmax, const SkipRule& skip, TraceHit& hit,
                                                         Stack stack, unsigned int* error_flag,
@@ -761,7 +824,7 @@ __device__ __forceinline__ bool traceAdvance(const DevScene& s, TraceState& q, c
     if constexpr (LOOP == kLoopQuery) {
         float tmax = q.tmax;
         TraceHit hit;
-        q.found = traceSceneOutOfLine<false, false>(s, q.origin, q.dir, q.tmin, tmax, skip, hit, stack,
+        q.found = traceSceneOutOfLine<false, false, false>(s, q.origin, q.dir, q.tmin, tmax, skip, hit, stack,
                                                     error_flag, nullptr, any);
         if (q.found) {
             q.tmax = tmax;
@@ -772,11 +835,11 @@ __device__ __forceinline__ bool traceAdvance(const DevScene& s, TraceState& q, c
     q.settle(s);
     int step = kStepDescend;
     if constexpr (LOOP == kLoopOneStep) {
-        step = (q.ref & kLeafBit) == 0u ? nodeStep(s.nodes, q, stack, error_flag, counts)
+        step = (q.ref & kLeafBit) == 0u ? nodeStep<false>(s.nodes, q, stack, error_flag, counts)
                                         : leafStep(s, q, skip, stack, error_flag, counts, any);
     } else {
         while (step == kStepDescend && (q.ref & kLeafBit) == 0u) {
-            step = nodeStep(s.nodes, q, stack, error_flag, counts);
+            step = nodeStep<false>(s.nodes, q, stack, error_flag, counts);
         }
         if (step == kStepDescend) {
             step = leafStep(s, q, skip, stack, error_flag, counts, any);
@@ -802,7 +865,8 @@ __device__ __forceinline__ bool traceAdvance(const DevScene& s, TraceState& q, c
 // it: one more dependent load in front of every node fetch. Holding it measured
 // 2.7% faster in the megakernel (128 registers a thread) and 3-4% slower in the
 // wavefront's persistent kernels, whose 96-register budget then spills.
-template <bool HOLD, typename Stack>
+// PACKED is nodeStep's.
+template <bool HOLD, bool PACKED, typename Stack>
 __device__ __forceinline__ bool traceSceneBody(const DevScene& s, float3 origin, float3 dir, float tmin, float& tmax,
                                                const SkipRule& skip, TraceHit& hit, const Stack& stack,
                                                unsigned int* error_flag, TraversalCounts* counts, bool any)
@@ -821,7 +885,7 @@ __device__ __forceinline__ bool traceSceneBody(const DevScene& s, float3 origin,
     for (;;) {
         q.settle(s);
         const int step = (q.ref & kLeafBit) == 0u
-                             ? nodeStep(HOLD ? held_nodes : s.nodes, q, stack, error_flag, counts)
+                             ? nodeStep<PACKED>(HOLD ? held_nodes : s.nodes, q, stack, error_flag, counts)
                              : leafStep(s, q, skip, stack, error_flag, counts, any);
         if (step == kStepFinished || (step == kStepPop && !popNext(q, stack))) {
             break;
@@ -838,13 +902,13 @@ __device__ __forceinline__ bool traceSceneBody(const DevScene& s, float3 origin,
 // keeps the kernels that call it small enough for the instruction cache. COUNT
 // selects the copy that counts work (the counting kernels); the timed kernels'
 // copy has no counting code at all.
-template <bool COUNT, bool HOLD, typename Stack>
+template <bool COUNT, bool HOLD, bool PACKED, typename Stack>
 static __device__ __noinline__ bool traceSceneOutOfLine(const DevScene& s, float3 origin, float3 dir, float tmin,
                                                         float& tmax, const SkipRule& skip, TraceHit& hit,
                                                         Stack stack, unsigned int* error_flag,
                                                         TraversalCounts* counts, bool any)
 {
-    return traceSceneBody<HOLD>(s, origin, dir, tmin, tmax, skip, hit, stack, error_flag, COUNT ? counts : nullptr,
+    return traceSceneBody<HOLD, PACKED>(s, origin, dir, tmin, tmax, skip, hit, stack, error_flag, COUNT ? counts : nullptr,
                                 any);
 }
 
@@ -854,26 +918,26 @@ static __device__ __noinline__ bool traceSceneOutOfLine(const DevScene& s, float
 // it, but a larger kernel. Which is faster depends on the scene (the
 // megakernel's autotuner picks). COUNT adds the work counts into `counts`;
 // without it `counts` is ignored.
-template <bool INLINE = false, bool COUNT = false, typename Stack>
+template <bool INLINE = false, bool COUNT = false, bool PACKED = false, typename Stack>
 ALB_DEV bool traceQuery(const DevScene& s, float3 origin, float3 dir, float tmin, float& tmax, const SkipRule& skip,
                         TraceHit& hit, const Stack& stack, unsigned int* error_flag, TraversalCounts* counts,
                         bool any)
 {
     if constexpr (INLINE) {
-        return traceSceneBody<true>(s, origin, dir, tmin, tmax, skip, hit, stack, error_flag,
+        return traceSceneBody<true, PACKED>(s, origin, dir, tmin, tmax, skip, hit, stack, error_flag,
                                     COUNT ? counts : nullptr, any);
     } else {
-        return traceSceneOutOfLine<COUNT, true>(s, origin, dir, tmin, tmax, skip, hit, stack, error_flag, counts,
+        return traceSceneOutOfLine<COUNT, true, PACKED>(s, origin, dir, tmin, tmax, skip, hit, stack, error_flag, counts,
                                                 any);
     }
 }
 
-template <bool ANY, bool INLINE = false, bool COUNT = false, typename Stack>
+template <bool ANY, bool INLINE = false, bool COUNT = false, bool PACKED = false, typename Stack>
 ALB_DEV bool traceScene(const DevScene& s, float3 origin, float3 dir, float tmin, float& tmax, const SkipRule& skip,
                         TraceHit& hit, const Stack& stack, unsigned int* error_flag,
                         TraversalCounts* counts = nullptr)
 {
-    return traceQuery<INLINE, COUNT>(s, origin, dir, tmin, tmax, skip, hit, stack, error_flag, counts, ANY);
+    return traceQuery<INLINE, COUNT, PACKED>(s, origin, dir, tmin, tmax, skip, hit, stack, error_flag, counts, ANY);
 }
 
 } // namespace albedo_b200
