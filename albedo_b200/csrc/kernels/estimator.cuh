@@ -226,7 +226,7 @@ ALB_DEV bool pathBounce(const DevScene& s, const Ctx& c, PathState& p, Pcg32& g,
         return false;
     }
     Surface sf;
-    resolveHit(s, p.o, p.d, hit, sf);
+    resolveHit<true>(s, p.o, p.d, hit, sf);
     p.result = p.result + p.throughput * weightedEmission(s, p, sf);
     if (p.depth >= max_depth) {
         return false;
@@ -247,7 +247,7 @@ ALB_DEV bool scatterOnlyBounce(const DevScene& s, const Ctx& c, PathState& p, Pc
         return false;
     }
     Surface sf;
-    resolveHit(s, p.o, p.d, hit, sf);
+    resolveHit<true>(s, p.o, p.d, hit, sf);
     const int light_index = s.object_light[sf.object_id];
     if (light_index >= 0 && sf.front) {
         p.result = p.result + p.throughput * ld3(s.lights[light_index].e);
@@ -279,7 +279,7 @@ ALB_DEV bool normalsBounce(const DevScene& s, const Ctx& c, PathState& p)
     TraceHit hit;
     if (closestHit(s, c, p.o, p.d, SkipRule::none(), hit)) {
         Surface sf;
-        resolveHit(s, p.o, p.d, hit, sf);
+        resolveHit<true>(s, p.o, p.d, hit, sf);
         p.result = mk(0.5f * (sf.ns.x + 1.0f), 0.5f * (sf.ns.y + 1.0f), 0.5f * (sf.ns.z + 1.0f));
     } else {
         const float h = 0.5f * (normalized(p.d).y + 1.0f);

@@ -53,30 +53,37 @@ ALB_DEV float3 blendedNormal(const DevTriangle& tri, const DevTriangleAttr& at, 
 }
 
 // The reported hit's distance recomputed once in FP64 (traversal decided which
-// primitive is nearest in FP32): the sphere root closest to the FP32 one, or the
-// watertight triangle distance, with instance rays taken to object space in FP64.
+// primitive is nearest in FP32): the sphere root closest to the FP32 one.
+ALB_DEV double refinedSphereDistance(const DevSphere& sp, float3 origin, float3 dir, const TraceHit& h)
+{
+    const double ox = origin.x, oy = origin.y, oz = origin.z;
+    const double dx = dir.x, dy = dir.y, dz = dir.z;
+    const double cx = ox - sp.cx, cy = oy - sp.cy, cz = oz - sp.cz;
+    const double a = dx * dx + dy * dy + dz * dz;
+    const double hh = dx * cx + dy * cy + dz * cz;
+    const double r2 = static_cast<double>(sp.r) * sp.r;
+    const double c = (cx * cx + cy * cy + cz * cz) - r2;
+    const double k = hh / a;
+    const double lx = cx - dx * k, ly = cy - dy * k, lz = cz - dz * k;
+    const double disc = fmax(a * (r2 - (lx * lx + ly * ly + lz * lz)), 0.0);
+    const double q = -(hh + copysign(sqrt(disc), hh));
+    if (q == 0.0) {
+        return 0.0;
+    }
+    const double r0 = q / a;
+    const double r1 = c / q;
+    return fabs(r0 - h.t) < fabs(r1 - h.t) ? r0 : r1;
+}
+
+// The same for any hit: the sphere root, or the watertight triangle distance,
+// with instance rays taken to object space in FP64.
 ALB_DEV double refinedDistance(const DevScene& s, float3 origin, float3 dir, const TraceHit& h)
 {
     const DevObject obj = s.objects[h.obj_pos];
     const double ox = origin.x, oy = origin.y, oz = origin.z;
     const double dx = dir.x, dy = dir.y, dz = dir.z;
     if (obj.kind == kObjSphere || obj.kind == kObjSphereWide) {
-        const DevSphere sp = s.spheres[obj.index];
-        const double cx = ox - sp.cx, cy = oy - sp.cy, cz = oz - sp.cz;
-        const double a = dx * dx + dy * dy + dz * dz;
-        const double hh = dx * cx + dy * cy + dz * cz;
-        const double r2 = static_cast<double>(sp.r) * sp.r;
-        const double c = (cx * cx + cy * cy + cz * cz) - r2;
-        const double k = hh / a;
-        const double lx = cx - dx * k, ly = cy - dy * k, lz = cz - dz * k;
-        const double disc = fmax(a * (r2 - (lx * lx + ly * ly + lz * lz)), 0.0);
-        const double q = -(hh + copysign(sqrt(disc), hh));
-        if (q == 0.0) {
-            return 0.0;
-        }
-        const double r0 = q / a;
-        const double r1 = c / q;
-        return fabs(r0 - h.t) < fabs(r1 - h.t) ? r0 : r1;
+        return refinedSphereDistance(s.spheres[obj.index], origin, dir, h);
     }
     double px = ox, py = oy, pz = oz, qx = dx, qy = dy, qz = dz;
     if (obj.kind == kObjInstance) {
@@ -117,6 +124,15 @@ ALB_DEV double refinedDistance(const DevScene& s, float3 origin, float3 dir, con
 }
 
 // Scene::intersect's record (scene/scene.cpp:107-133) for a TraceHit.
+//
+// SPHERE computes a sphere hit's distance with the sphere's formula alone; without
+// it the general form is compiled in, whose triangle half a sphere never runs.
+// The megakernel takes the short form: 5 KB less of a kernel whose top stall is
+// instruction fetch, and 56 bytes less of frame. The wavefront's shade kernels
+// and the ray queries keep the general one: their compiler contracts the short
+// form's products otherwise, their images would change in the last place, and
+// they do not gain (trefoils 49.3 and 49.5 ms).
+template <bool SPHERE = false>
 ALB_DEV void resolveHit(const DevScene& s, float3 origin, float3 dir, const TraceHit& h, Surface& out)
 {
     const DevObject obj = s.objects[h.obj_pos];
@@ -132,7 +148,8 @@ ALB_DEV void resolveHit(const DevScene& s, float3 origin, float3 dir, const Trac
     if (obj.kind == kObjSphere || obj.kind == kObjSphereWide) {
         const DevSphere sp = s.spheres[obj.index];
         // The hit point from the FP64 distance: FP32 o + t d loses the walls' 1e4-scale digits.
-        const double t = refinedDistance(s, origin, dir, h);
+        const double t =
+            SPHERE ? refinedSphereDistance(sp, origin, dir, h) : refinedDistance(s, origin, dir, h);
         out.p = mk(static_cast<float>(origin.x + dir.x * t), static_cast<float>(origin.y + dir.y * t),
                    static_cast<float>(origin.z + dir.z * t));
         n = normalized(mk(static_cast<float>(origin.x + dir.x * t - sp.cx),
@@ -341,7 +358,11 @@ struct Ggx {
 
 // Unpolarized reflectance at a smooth boundary with a real relative index
 // (scattering/fresnel.cpp:17-47; the complex form with zero imaginary part).
-ALB_DEV float fresnelDielectric(float cos_i, float eta)
+// Out of line: five divisions at four places of the megakernel were 8 KB of
+// it. With the short sphere form of resolveHit, ms: sphere room 8.17 -> 7.68,
+// trefoils 269.0 -> 265.3, icosphere 179.3 -> 175.2, the room's scatter-only
+// estimator at 1174x843 172.4 -> 162.8; the wavefront is unchanged.
+static __device__ __noinline__ float fresnelDielectric(float cos_i, float eta)
 {
     if (cos_i < 0.0f) {
         cos_i = -cos_i;
