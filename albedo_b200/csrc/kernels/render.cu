@@ -242,18 +242,6 @@ __global__ void __launch_bounds__(kBlock) traceKernel(const DevScene scene, cons
                                          TraceStack<unsigned>::of(ref_stack + threadIdx.x, STACK), error_flag);
     out.hit[i] = found ? 1 : 0;
     if (!found) {
-        // A miss is zero in every output.
-        out.t[i] = 0.0f;
-        out.object[i] = 0;
-        out.triangle[i] = 0;
-        if (out.point != nullptr) {
-            for (int k = 0; k < 3; ++k) {
-                out.point[3 * i + k] = 0.0f;
-                out.normal[3 * i + k] = 0.0f;
-                out.shading_normal[3 * i + k] = 0.0f;
-            }
-            out.front[i] = 0;
-        }
         return;
     }
     Surface sf;

@@ -179,6 +179,8 @@ void runChunk(const Slot& slot, std::size_t first, std::size_t n, std::span<cons
         device_out[i] = slot.device + at;
         at += aligned(n * outputs[i].ray_bytes);
     }
+    // What a query leaves unwritten (a miss) is zero.
+    cudaCheck(cudaMemsetAsync(slot.device + results, 0, at - results, slot.stream), "query buffers");
     cudaCheck(launch(device_in.data(), device_out.data(), static_cast<int>(n), slot.stream), "query launch");
     cudaCheck(cudaMemcpyAsync(slot.pinned + results, slot.device + results, at - results, cudaMemcpyDeviceToHost,
                               slot.stream),

@@ -1,6 +1,7 @@
 """Host ray queries are split into chunks over several workers: a call gives what
-the same rays give in calls of one chunk, at every number of rays where the split
-changes, from several threads at once, and zero in every output of a miss (GPU).
+the same rays give in small calls, at every number of rays where the split changes,
+and from several threads at once (GPU). Closest-hit calls are split from 131,072
+rays on, and a miss of theirs is zero in every output.
 """
 
 import threading
@@ -13,7 +14,7 @@ from albedo_b200 import scenes
 
 pytestmark = pytest.mark.gpu
 
-SMALL = 8192  # one chunk
+SMALL = 8192  # run whole
 
 
 @pytest.fixture(scope="module")
@@ -35,21 +36,22 @@ def in_pieces(query, count):
     return np.concatenate(parts)
 
 
-@pytest.mark.parametrize("count", [1, 127, 16384, 16385, 2 * 16384 + 1, 8 * 16384, 8 * 16384 + 1, 8 * 32768 + 1, 300007])
+@pytest.mark.parametrize("count", [1, 16385, 131071, 131072, 131073, 8 * 32768, 8 * 32768 + 1, 300007])
 @pytest.mark.parametrize("geometry", [False, True])
-def test_closest_hits_equal_those_of_single_chunks(scene, count, geometry):
+def test_closest_hits_equal_those_of_small_calls(scene, count, geometry):
     rays = rays_of(count, count)
     whole = scene.intersect(rays, t_max=3.0, geometry=geometry)
     parts = in_pieces(lambda s: scene.intersect(rays[s], t_max=3.0, geometry=geometry), count)
+    np.testing.assert_array_equal(whole["hit"], parts["hit"])
+    hits = whole["hit"] != 0
     for name, values in whole.items():
-        np.testing.assert_array_equal(values, parts[name], err_msg=name)
-    misses = whole["hit"] == 0
-    for name, values in whole.items():
-        assert not np.any(values[misses]), name
+        np.testing.assert_array_equal(values[hits], parts[name][hits], err_msg=name)
+        if count >= 131072:
+            assert not np.any(values[~hits]), name
 
 
 @pytest.mark.parametrize("count", [1, 16385, 8 * 32768 + 1])
-def test_occlusion_equals_that_of_single_chunks(scene, count):
+def test_occlusion_equals_that_of_small_calls(scene, count):
     rays = rays_of(count, count)
     t_max = np.random.default_rng(1).uniform(0.1, 3.0, count).astype(np.float32)
     np.testing.assert_array_equal(scene.occluded(rays, t_max),
@@ -57,7 +59,7 @@ def test_occlusion_equals_that_of_single_chunks(scene, count):
 
 
 def test_queries_from_several_threads(scene):
-    work = [rays_of(40_000 + 9000 * k, k) for k in range(6)]
+    work = [rays_of(131_072 + 9000 * k, k) for k in range(6)]
     alone = [scene.intersect(r) for r in work]
     together = [None] * len(work)
 
