@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) extendKernel(const WfJ
     const WfSlots& sl = b.slots;
     const auto lane_stack = TraceStack<unsigned>::of(ref_stack + threadIdx.x, STACK);
     const int lanes = raysPerWarp(count);
-    WarpFetch fetch{0, 0, min(fetch_batch, lanes), false};
+    WarpFetch fetch{0, 0, lanes < 32 ? lanes : fetch_batch, false};
     const bool takes = static_cast<int>(threadIdx.x & 31u) < lanes;
     TraceState q;
     SkipRule skip = SkipRule::none();
@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSm) shadowKernel(const WfJ
     const WfSlots& sl = b.slots;
     const auto lane_stack = TraceStack<unsigned>::of(ref_stack + threadIdx.x, STACK);
     const int lanes = raysPerWarp(count);
-    WarpFetch fetch{0, 0, min(fetch_batch, lanes), false};
+    WarpFetch fetch{0, 0, lanes < 32 ? lanes : fetch_batch, false};
     const bool takes = static_cast<int>(threadIdx.x & 31u) < lanes;
     TraceState q;
     SkipRule skip = SkipRule::none();
