@@ -817,6 +817,12 @@ cudaError_t wfIteration(const WfJob* jobs, const WfBuffers& b, const WfLaunch& l
     const int fetch = launch.fetch_batch > 0 ? launch.fetch_batch : 32;
     // The persistent traversal kernels keep 4-byte stack entries (references only).
     const auto smemFor = [](int entries) { return static_cast<std::size_t>(entries) * 128 * sizeof(unsigned); };
+    // The four shade kernels run beside each other, and each leaves room for the
+    // others at three blocks per SM of the default four: trefoil frame at 16
+    // samples 46.8 ms against 49.3 at four and 49.7 at eight, 16-job batch 102.4 /
+    // 103.4 / 104.1, sphere room 8.2 / 8.3 / 8.5; two are slower again (47.7, 103.3,
+    // 8.3).
+    const int sg = g >= 4 ? g / 4 * 3 : g;
     regenKernel<<<g, 128, 0, stream>>>(jobs, b);
     const bool binned = launch.ray_sort != 0 && b.binned != nullptr;
     if (binned) {
@@ -843,10 +849,10 @@ cudaError_t wfIteration(const WfJob* jobs, const WfBuffers& b, const WfLaunch& l
         if (e != cudaSuccess) {
             return e;
         }
-        shadeKernel<kClassDiffuse><<<g, 128, 0, stream>>>(jobs, b);
-        shadeKernel<kClassConductor><<<g, 128, 0, side->stream[0]>>>(jobs, b);
-        shadeKernel<kClassDielectric><<<g, 128, 0, side->stream[1]>>>(jobs, b);
-        shadeKernel<kClassMix><<<g, 128, 0, side->stream[2]>>>(jobs, b);
+        shadeKernel<kClassDiffuse><<<sg, 128, 0, stream>>>(jobs, b);
+        shadeKernel<kClassConductor><<<sg, 128, 0, side->stream[0]>>>(jobs, b);
+        shadeKernel<kClassDielectric><<<sg, 128, 0, side->stream[1]>>>(jobs, b);
+        shadeKernel<kClassMix><<<sg, 128, 0, side->stream[2]>>>(jobs, b);
         for (int k = 0; k < 3 && e == cudaSuccess; ++k) {
             e = cudaEventRecord(side->join[k], side->stream[k]);
             if (e == cudaSuccess) {
@@ -857,10 +863,10 @@ cudaError_t wfIteration(const WfJob* jobs, const WfBuffers& b, const WfLaunch& l
             return e;
         }
     } else {
-        shadeKernel<kClassDiffuse><<<g, 128, 0, stream>>>(jobs, b);
-        shadeKernel<kClassConductor><<<g, 128, 0, stream>>>(jobs, b);
-        shadeKernel<kClassDielectric><<<g, 128, 0, stream>>>(jobs, b);
-        shadeKernel<kClassMix><<<g, 128, 0, stream>>>(jobs, b);
+        shadeKernel<kClassDiffuse><<<sg, 128, 0, stream>>>(jobs, b);
+        shadeKernel<kClassConductor><<<sg, 128, 0, stream>>>(jobs, b);
+        shadeKernel<kClassDielectric><<<sg, 128, 0, stream>>>(jobs, b);
+        shadeKernel<kClassMix><<<sg, 128, 0, stream>>>(jobs, b);
     }
     // The shadow rays too, when binning is 2. The binned buffer is free again:
     // the extend kernel has read it.
