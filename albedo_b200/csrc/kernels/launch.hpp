@@ -50,8 +50,8 @@ enum Accumulation : int { kAccumulateFp64 = 0, kAccumulateKahan = 1 };
 // the scene's hierarchy is deeper than every compiled variant supports.
 int stackCapacityFor(std::uint32_t stack_need);
 
-// Traversal-stack capacities the kernels are compiled for (8 bytes per entry per
-// thread of shared memory; 48 entries keep four 128-thread blocks per SM).
+// Traversal-stack capacities the kernels are compiled for (4 bytes per entry per
+// thread of shared memory, 24 KB a block of 128 threads at 48 entries).
 template <int S>
 struct StackSize {
     static constexpr int value = S;

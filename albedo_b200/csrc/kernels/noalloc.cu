@@ -7,7 +7,7 @@
 //
 // The array is sized for kNoAllocMaxSlots path slots, one per pixel, so images
 // of at most 65,536 pixels fit; larger ones are rejected. Every GPU that loads
-// the library holds the array (about 17 MB) until the process exits. Every call
+// the library holds the array (about 15 MB) until the process exits. Every call
 // shares it and it keeps the last call's contents: each call clears what must
 // start at zero (queues, counters, slot ownership) before use, and calls whose
 // work overlaps on the GPU race on it, so callers must not overlap them.

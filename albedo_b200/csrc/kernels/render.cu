@@ -3,9 +3,10 @@
 // renderPixel (render/render_image.cpp:27-44): each pixel owns one PCG32 stream
 // and draws its n x n stratified samples from it in row-major order, so one
 // thread runs one pixel's samples serially. Blocks cover tiles of 128 pixels
-// (16 x 8 by default) so a warp's camera rays start coherent. The traversal stack of every thread sits in
-// shared memory: STACK child references of 4 bytes, or STACK entries of 8 bytes
-// in the counting kernels.
+// (16 x 8 by default; fewer pixels for small images) so a warp's camera rays start
+// coherent. The traversal stack of every thread sits in shared memory: STACK
+// child references of 4 bytes, or STACK entries of 8 bytes in the counting
+// kernels.
 #include "estimator.cuh"
 
 #include <type_traits>
@@ -17,9 +18,11 @@ namespace {
 constexpr int kBlock = kTraceBlock;
 constexpr int kTileW = 16; // default tile: 16 x 8 pixels
 // Resident blocks per SM the megakernel's register budget is sized for by
-// default: 3 (168 registers a thread) measured 4-12% faster than 4 (128
-// registers, with local-memory spills) on the room and trefoil scenes. The
-// path estimator is also compiled for 4; the autotuner picks per scene.
+// default: 3 (168 registers a thread). The path estimator is also compiled for 4
+// (128 registers, lean), which wins where traversal dominates (1.31M-triangle
+// icosphere 175.6 -> 154.0 ms, soup 49.1 -> 43.2, trefoils 264.8 -> 254.8) and
+// loses where shading does (sphere room 7.68 -> 8.09, meshes among mixed
+// materials up to 30.3 -> 33.7): the autotuner picks per scene.
 #ifndef ALBEDO_MEGA_BLOCKS_PER_SM
 #define ALBEDO_MEGA_BLOCKS_PER_SM 3
 #endif

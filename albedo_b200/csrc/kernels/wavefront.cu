@@ -61,7 +61,7 @@ ALB_DEV unsigned long long claimItem(unsigned long long* next, bool want)
 }
 
 // Resident blocks per SM the traversal kernels' register budget is sized for:
-// 5 (96 registers a thread, no spills). With 4-byte stack entries five blocks'
+// 5 (96 registers a thread, tens of bytes of spills). With 4-byte stack entries five blocks'
 // stacks fit in shared memory; 5 measured 6-10% faster than 4 on the trefoil,
 // icosphere and 64-job workloads.
 #ifndef ALBEDO_TRACE_BLOCKS_PER_SM

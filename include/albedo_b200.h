@@ -225,7 +225,7 @@ int albedo_render_batch(const albedo_batch_item* items, int32_t count, void* str
  * allocator owns up front (a framework's caching pool that has reserved the
  * GPU), or a loop with a latency budget, where an allocation can stall on the
  * driver or synchronize the device. The wavefront's path slots, queues and
- * control block live in a static device array of about 17 MB that every GPU
+ * control block live in a static device array of about 15 MB that every GPU
  * loading the library holds until exit. It holds one path slot per pixel, so
  * images are limited to 65,536 pixels; larger ones are rejected with
  * ALBEDO_INVALID_ARGUMENT. The first call on a device looks up that array's
