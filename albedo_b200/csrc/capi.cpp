@@ -312,6 +312,10 @@ struct albedo_scene {
         dev.world_triangles = host.triangles.empty() ? 0u : 1u;
         error_flag = DeviceBuffer{sizeof(unsigned int)};
         check(cudaMemset(error_flag.ptr, 0, sizeof(unsigned int)), "cudaMemset");
+        // Copies from pageable memory and the memset may return before the device
+        // has them; queries from host arrays run on streams that do not wait for
+        // the default one.
+        check(cudaStreamSynchronize(nullptr), "commit");
         int device{0};
         check(cudaGetDevice(&device), "cudaGetDevice");
         query_share.hold(device);
@@ -1654,10 +1658,30 @@ int albedo_scene_check(const albedo_scene* scene)
 
 namespace {
 
+// Throws for an array in device memory and, when `needed`, for a null one.
+void requireHostArray(const void* array, bool needed)
+{
+    if (array == nullptr) {
+        check(needed ? cudaErrorInvalidValue : cudaSuccess, "upload");
+        return;
+    }
+    cudaPointerAttributes at{};
+    check(cudaPointerGetAttributes(&at, array), "query array");
+    check(at.type == cudaMemoryTypeDevice ? cudaErrorInvalidValue : cudaSuccess, "query array");
+}
+
 // runQueries with its CUDA failures as device errors.
 void hostQueries(int64_t count, std::span<const QueryInput> inputs, std::span<const QueryOutput> outputs,
                  const QueryLaunch& launch)
 {
+    // The workers read and write the arrays with the host's own copies: what those
+    // cannot touch is refused, as a copy by the driver would have.
+    for (const QueryInput& in : inputs) {
+        requireHostArray(in.host, count > 0);
+    }
+    for (const QueryOutput& out : outputs) {
+        requireHostArray(out.host, false);
+    }
     try {
         runQueries(count, inputs, outputs, launch);
     } catch (const std::bad_alloc&) {
