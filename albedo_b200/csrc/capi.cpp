@@ -391,6 +391,7 @@ RenderArgs renderArgsFor(const albedo_scene& scene, const albedo_render_job& job
     args.roulette_start = job.roulette_start;
     args.tile_width = scene.mega_tile_width;
     args.blocks_per_sm = scene.mega_blocks_per_sm;
+    args.mesh_steps = scene.image.mesh_steps;
     args.accumulation = job.accumulation;
     // The inlined-traversal kernel exists for the path estimator; the other
     // estimators keep the out-of-line traversal (images do not depend on it).

@@ -330,6 +330,41 @@ void checkFp32Range(const DeviceImage& image)
 
 } // namespace
 
+namespace {
+
+double halfArea(double x, double y, double z)
+{
+    return x * y + y * z + z * x;
+}
+
+// Nodes of nodes[first ..] a line through the root's box is expected to enter: a
+// uniformly random line that enters a convex body enters a box inside it with the
+// ratio of their surface areas (Goldsmith and Salmon 1987).
+float expectedNodeSteps(const std::vector<DevNode>& nodes, std::size_t first, std::uint32_t root)
+{
+    if (first == nodes.size() || root == kEmptyChild) {
+        return 0.0f;
+    }
+    const DevNode& top{nodes[root]};
+    const auto extent = [&](const float* lo, const float* hi) {
+        return static_cast<double>(*std::max_element(hi, hi + top.count)) - *std::min_element(lo, lo + top.count);
+    };
+    const double whole{halfArea(extent(top.lo_x, top.hi_x), extent(top.lo_y, top.hi_y), extent(top.lo_z, top.hi_z))};
+    double sum{0.0};
+    for (std::size_t i{first}; i < nodes.size(); ++i) {
+        const DevNode& n{nodes[i]};
+        for (std::uint32_t c{0}; c < n.count; ++c) {
+            if ((n.child[c] & kLeafBit) == 0u) {
+                sum += halfArea(static_cast<double>(n.hi_x[c]) - n.lo_x[c], static_cast<double>(n.hi_y[c]) - n.lo_y[c],
+                                static_cast<double>(n.hi_z[c]) - n.lo_z[c]);
+            }
+        }
+    }
+    return whole > 0.0 ? static_cast<float>(1.0 + sum / whole) : 0.0f;
+}
+
+} // namespace
+
 DeviceImage flattenScene(const HostScene& scene)
 {
     DeviceImage image;
@@ -341,6 +376,7 @@ DeviceImage flattenScene(const HostScene& scene)
         image.attrs.push_back(deviceAttr(scene.triangles[i], nullptr));
     }
     std::vector<std::uint32_t> mesh_root(scene.meshes.size(), kEmptyChild);
+    std::vector<float> mesh_steps(scene.meshes.size(), 0.0f);
     std::uint32_t max_blas_need{0};
     for (std::size_t m{0}; m < scene.meshes.size(); ++m) {
         const MeshDesc& mesh{scene.meshes[m]};
@@ -373,7 +409,9 @@ DeviceImage flattenScene(const HostScene& scene)
         for (std::jthread& worker : workers) {
             worker.join();
         }
+        const std::size_t first_node{image.nodes.size()};
         const Emitted blas{emitBvh(mesh.bvh, base, image.nodes)};
+        mesh_steps[m] = expectedNodeSteps(image.nodes, first_node, blas.root);
         mesh_root[m] = blas.root;
         max_blas_need = std::max(max_blas_need, blas.stack_need);
     }
@@ -424,6 +462,7 @@ DeviceImage flattenScene(const HostScene& scene)
         putAffine(d.to_object, inst.to_object.forward());
         putAffine(d.to_world, inst.to_world.forward());
         d.root = mesh_root[inst.mesh];
+        image.mesh_steps = std::max(image.mesh_steps, mesh_steps[inst.mesh]);
         d.mesh = inst.mesh;
         image.instances.push_back(d);
         const Affine& back{inst.to_object.forward()};

@@ -35,6 +35,8 @@ struct DeviceImage {
     std::int32_t sky_light{-1};
     // Traversal stack entries a query can need: TLAS depth + deepest BLAS + 2.
     std::uint32_t stack_need{0};
+    // Nodes a ray through the box of the costliest instanced mesh is expected to enter.
+    float mesh_steps{0.0f};
 };
 
 // Throws std::invalid_argument if the scene exceeds the device layout's limits

@@ -30,7 +30,8 @@ struct RenderArgs {
     double* sum_squares; // optional per-pixel (or per-listed-pixel) sums of squared samples, 3 doubles each
     // Launch shape of the megakernel (the autotuner's knobs): pixel tile width
     // (8, 16 or 32; tiles hold 128 pixels) and register budget (resident blocks
-    // per SM the kernel is compiled for: 3 or 4). 0 picks the default (16, 3).
+    // per SM the kernel is compiled for: 3 or 4). 0 picks the default (16; 3 or 4
+    // by the image's size and the meshes' query cost).
     int tile_width;
     int blocks_per_sm;
     // Lanes of each warp that take a pixel (1, 2, 4, ..., 32); the launcher sets it.
@@ -42,6 +43,9 @@ struct RenderArgs {
     // (compensated FP32, path estimator only). Either is added to the FP64
     // accumulators at the end.
     int accumulation;
+    // Nodes a ray through the box of the scene's costliest mesh is expected to
+    // enter (the launcher's choice of blocks_per_sm 0 reads it).
+    float mesh_steps;
 };
 
 enum Accumulation : int { kAccumulateFp64 = 0, kAccumulateKahan = 1 };

@@ -17,12 +17,10 @@ namespace {
 
 constexpr int kBlock = kTraceBlock;
 constexpr int kTileW = 16; // default tile: 16 x 8 pixels
-// Resident blocks per SM the megakernel's register budget is sized for by
-// default: 3 (168 registers a thread). The path estimator is also compiled for 4
-// (128 registers, lean), which wins where traversal dominates (1.31M-triangle
-// icosphere 175.6 -> 154.0 ms, soup 49.1 -> 43.2, trefoils 264.8 -> 254.8) and
-// loses where shading does (sphere room 7.68 -> 8.09, meshes among mixed
-// materials up to 30.3 -> 33.7): the autotuner picks per scene.
+// Resident blocks per SM the megakernel's register budget is sized for: 3 (168
+// registers a thread). The path estimator is also compiled for 4 (128 registers,
+// lean); chooseBlocksPerSm says when each is taken for a scene that has not been
+// tuned.
 #ifndef ALBEDO_MEGA_BLOCKS_PER_SM
 #define ALBEDO_MEGA_BLOCKS_PER_SM 3
 #endif
@@ -335,6 +333,11 @@ cudaError_t spreadOver(int warps_per_sm, long long items, int& lanes)
     return e;
 }
 
+long long imagePixels(const RenderArgs& args)
+{
+    return args.pixels != nullptr ? args.pixel_count : static_cast<long long>(args.width) * args.height;
+}
+
 // How many lanes of a warp take a pixel (RenderArgs::warp_pixels): 32, or fewer
 // for an image too small to fill the GPU with full warps. A pixel's samples run
 // in sequence on its lane, so a small image takes as long as its slowest warps,
@@ -357,9 +360,45 @@ cudaError_t spreadOver(int warps_per_sm, long long items, int& lanes)
 cudaError_t chooseWarpPixels(const DevScene& scene, RenderArgs& args)
 {
     constexpr std::uint32_t kFewTriangles = 256;
-    const long long pixels =
-        args.pixels != nullptr ? args.pixel_count : static_cast<long long>(args.width) * args.height;
-    return spreadOver(scene.triangle_count < kFewTriangles ? 3 : 12, pixels, args.warp_pixels);
+    return spreadOver(scene.triangle_count < kFewTriangles ? 3 : 12, imagePixels(args), args.warp_pixels);
+}
+
+// The register budget of a path-estimator launch that names none: 4 blocks per SM
+// (lean) for images of many waves of warps, 3 otherwise. Four resident warps a
+// scheduler hide more of a query's dependent fetches than three, but each warp then
+// takes longer over its pixels' samples, which run in sequence. With many waves the
+// longer chains of a few pixels are overlapped by other warps; with few, the launch
+// waits for them. A mesh whose queries enter many nodes (overlapping boxes:
+// RenderArgs::mesh_steps) waits longest on memory and gains from fewer waves on.
+//
+// Measured, lean over 3 blocks per SM: 1920x1080, 36 waves of the 3-block shape, in
+// 25 scenes of 5 to 1.31M triangles and one to seven materials, 2 and 3 samples an
+// axis, 0.84 (200,003-triangle soup) to 0.98 (instances of gold and rough glass);
+// 1440x810, 20 waves: 0.90 to 1.01; 1280x720, 16 waves: 0.84 to 1.02; 960x540, 9
+// waves: 0.89 to 1.05; 640x360, 4 waves: up to 1.11. Soups of 20,000 to 300,000
+// triangles (mesh_steps 43 to 221) take 0.80 to 0.92 from 800x450, 6.3 waves, on,
+// but up to 1.06 at 640x360. Closed surfaces of 1,280 to 1.31M triangles (12 to 24)
+// scatter between 0.92 and 1.08 at 800x450.
+constexpr int kDefaultWarpsPerSm = kMegaBlocksPerSm * kBlock / 32;
+
+cudaError_t chooseBlocksPerSm(RenderArgs& args)
+{
+    if (args.blocks_per_sm != 0 || args.estimator != kEstimatorPath) {
+        return cudaSuccess;
+    }
+    constexpr int kManyWaves = 20;
+    constexpr int kCostlyMeshWaves = 6;
+    constexpr float kCostlyMeshSteps = 40.0f;
+    const int waves = args.mesh_steps >= kCostlyMeshSteps ? kCostlyMeshWaves : kManyWaves;
+    int device = 0;
+    int sms = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) {
+        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    }
+    const long long full = static_cast<long long>(sms) * kDefaultWarpsPerSm * args.warp_pixels * waves;
+    args.blocks_per_sm = imagePixels(args) >= full ? 4 : kMegaBlocksPerSm;
+    return e;
 }
 
 // Ray queries spread likewise, over 8 warps per SM (a staged call runs up to eight
@@ -450,7 +489,10 @@ cudaError_t launchMegakernel(const DevScene& scene, const DevCamera& camera, con
                              PixelAccum* accum, unsigned int* error_flag, int stack_capacity, cudaStream_t stream)
 {
     RenderArgs args = render;
-    const cudaError_t chosen = chooseWarpPixels(scene, args);
+    cudaError_t chosen = chooseWarpPixels(scene, args);
+    if (chosen == cudaSuccess) {
+        chosen = chooseBlocksPerSm(args);
+    }
     if (chosen != cudaSuccess) {
         return chosen;
     }

@@ -323,7 +323,9 @@ int albedo_wavefront_configure(int32_t slot_count, int32_t blocks_per_sm, int32_
 typedef struct albedo_tuning {
     int32_t tile_width;           /* megakernel: pixel tile width (8, 16 or 32; 128-pixel tiles) */
     int32_t blocks_per_sm;        /* megakernel: register budget (3 or 4 resident blocks per SM; at 4
-                                     the path estimator keeps each path's state in shared memory);
+                                     the path estimator keeps each path's state in shared memory;
+                                     a scene without a shape of its own takes 3, or 4 for large
+                                     images, and reads 3 here);
                                      wavefront: blocks per SM of the queue kernels */
     int32_t trace_blocks_per_sm;  /* wavefront: persistent traversal blocks per SM */
     int32_t fetch_batch;          /* wavefront: queue entries a traversal warp claims at once */
