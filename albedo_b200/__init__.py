@@ -285,7 +285,8 @@ class Scene:
 
     # Ray queries.
     def intersect(self, rays: np.ndarray, t_min: float = 0.0, t_max: float = float("inf"), geometry: bool = False):
-        """Closest hits of (N, 6) float32 rays: dict of hit, t, object, triangle [, point, normal, ...]."""
+        """Closest hits of (N, 6) float32 rays: dict of hit, t, object, triangle [, point, normal, ...].
+        A miss is zero in all of them."""
         rays = np.ascontiguousarray(rays, dtype=np.float32).reshape(-1, 6)
         n = len(rays)
         out = {"hit": np.zeros(n, np.int32), "t": np.zeros(n, np.float32), "object": np.full(n, -1, np.int32),

@@ -1692,14 +1692,9 @@ void hostQueries(int64_t count, std::span<const QueryInput> inputs, std::span<co
     }
 }
 
-// Closest-hit calls of this many rays and more are staged in chunks. Smaller ones
-// run as one launch over buffers of the call's own: a miss writes its hit flag
-// alone, so its other outputs are what the new buffers held, and that is left as
-// it was. Buffers of a large call come zeroed, so there a miss is zero, staged
-// or not. 131,072 rays with geometry take 4.9 ms whole and 2.0 staged.
-constexpr int64_t kStagedTraceRays{1 << 17};
-
-void traceStaged(const albedo_scene& scene, const float* rays, int64_t count, float t_min, float t_max, int32_t* hit,
+// A miss writes its hit flag alone; its other outputs are the zeros its chunk's
+// buffers start with (runQueries), at every number of rays.
+void closestHits(const albedo_scene& scene, const float* rays, int64_t count, float t_min, float t_max, int32_t* hit,
                  float* t, int32_t* object, int32_t* triangle, float* point, float* normal, float* shading_normal,
                  int32_t* front)
 {
@@ -1725,39 +1720,6 @@ void traceStaged(const albedo_scene& scene, const float* rays, int64_t count, fl
     });
 }
 
-void traceWhole(const albedo_scene& scene, const float* rays, int64_t count, float t_min, float t_max, int32_t* hit,
-                float* t, int32_t* object, int32_t* triangle, float* point, float* normal, float* shading_normal,
-                int32_t* front)
-{
-    const auto n{static_cast<std::size_t>(count)};
-    DeviceBuffer d_rays{uploadRaw(rays, 6 * n)};
-    DeviceBuffer d_hit{n * sizeof(int)};
-    DeviceBuffer d_t{n * sizeof(float)};
-    DeviceBuffer d_object{n * sizeof(int)};
-    DeviceBuffer d_triangle{n * sizeof(int)};
-    const bool geometry{point != nullptr};
-    DeviceBuffer d_point{geometry ? 3 * n * sizeof(float) : 0};
-    DeviceBuffer d_normal{geometry ? 3 * n * sizeof(float) : 0};
-    DeviceBuffer d_shading{geometry ? 3 * n * sizeof(float) : 0};
-    DeviceBuffer d_front{geometry ? n * sizeof(int) : 0};
-    TraceOutputs out{d_hit.as<int>(),   d_t.as<float>(),      d_object.as<int>(),   d_triangle.as<int>(),
-                     d_point.as<float>(), d_normal.as<float>(), d_shading.as<float>(), d_front.as<int>()};
-    check(launchTrace(scene.dev, d_rays.as<float>(), static_cast<int>(count), t_min, t_max, out,
-                      scene.error_flag.as<unsigned int>(), scene.stack_capacity, nullptr),
-          "trace launch");
-    check(cudaDeviceSynchronize(), "trace");
-    download(hit, d_hit, n);
-    download(t, d_t, n);
-    download(object, d_object, n);
-    download(triangle, d_triangle, n);
-    if (geometry) {
-        download(point, d_point, 3 * n);
-        download(normal, d_normal, 3 * n);
-        download(shading_normal, d_shading, 3 * n);
-        download(front, d_front, n);
-    }
-}
-
 } // namespace
 
 int albedo_trace_host(const albedo_scene* scene, const float* rays, int64_t count, float t_min, float t_max,
@@ -1766,13 +1728,7 @@ int albedo_trace_host(const albedo_scene* scene, const float* rays, int64_t coun
 {
     return guarded([&] {
         scene->requireCommitted();
-        if (count >= kStagedTraceRays) {
-            traceStaged(*scene, rays, count, t_min, t_max, hit, t, object, triangle, point, normal, shading_normal,
-                        front);
-        } else {
-            traceWhole(*scene, rays, count, t_min, t_max, hit, t, object, triangle, point, normal, shading_normal,
-                       front);
-        }
+        closestHits(*scene, rays, count, t_min, t_max, hit, t, object, triangle, point, normal, shading_normal, front);
         scene->collectKernelError();
     });
 }
