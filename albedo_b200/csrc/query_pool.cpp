@@ -217,6 +217,11 @@ void runQueries(std::int64_t count, std::span<const QueryInput> inputs, std::spa
     if (ray_bytes > kMaxQueryRayBytes || inputs.size() > kMaxQueryArrays || outputs.size() > kMaxQueryArrays) {
         throw std::logic_error{"a query takes more bytes a ray than a worker's buffers hold"};
     }
+    // The caller's arrays may still be filled, or read, by work on the default
+    // stream (and the streams that order themselves with it): pinned or managed
+    // memory takes asynchronous copies and kernels. The workers read and write the
+    // arrays on the host, so that work has to be over first.
+    cudaCheck(cudaStreamSynchronize(cudaStreamLegacy), "queries");
     int device{0};
     cudaCheck(cudaGetDevice(&device), "cudaGetDevice");
     DevicePool& pool{poolOf(device)};

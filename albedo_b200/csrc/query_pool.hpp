@@ -44,8 +44,9 @@ constexpr std::size_t kMaxQueryRayBytes{84};
 using QueryLaunch =
     std::function<cudaError_t(void* const* inputs, void* const* outputs, int count, cudaStream_t stream)>;
 
-// Runs `count` queries on the current device and returns when every result is
-// in its host array. Safe from several threads. Throws std::bad_alloc, or
+// Runs `count` queries on the current device, after the work that the default
+// stream held when the call was made, and returns when every result is in its
+// host array. Safe from several threads. Throws std::bad_alloc, or
 // std::runtime_error for any other CUDA failure.
 void runQueries(std::int64_t count, std::span<const QueryInput> inputs, std::span<const QueryOutput> outputs,
                 const QueryLaunch& launch);

@@ -391,7 +391,9 @@ int albedo_scene_check(const albedo_scene* scene);
 /* Ray queries over host arrays of rays (origin xyz, direction xyz as floats).
  * trace: hit flag, t, object id (add order), triangle id within its mesh (-1 if
  * none), and optionally point / normal / shading normal (3 floats each) and
- * front-face flags; a miss is zero in every output. occluded: any hit in (0, t_max[i]). */
+ * front-face flags; a miss is zero in every output. occluded: any hit in (0, t_max[i]).
+ * The arrays are read and written after the work that the default stream held at
+ * the call; work on non-blocking streams is the caller's to wait for. */
 int albedo_trace_host(const albedo_scene* scene, const float* rays, int64_t count, float t_min, float t_max,
                       int32_t* hit, float* t, int32_t* object, int32_t* triangle, float* point, float* normal,
                       float* shading_normal, int32_t* front);

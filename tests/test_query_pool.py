@@ -1,0 +1,37 @@
+"""The workers of host ray queries, on the host against a stand-in for the CUDA
+runtime (tests/cpp/query_pool.cpp)."""
+
+from __future__ import annotations
+
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+from albedo_b200.build import CSRC, _cuda_home
+
+HERE = Path(__file__).resolve().parent
+
+
+@pytest.fixture(scope="module")
+def exe(tmp_path_factory):
+    include = _cuda_home() / "include"
+    if shutil.which("g++") is None or not (include / "cuda_runtime_api.h").exists():
+        pytest.skip("g++ or the CUDA headers are not available")
+    out = tmp_path_factory.mktemp("pool") / "query_pool"
+    subprocess.run(["g++", "-std=c++20", "-O1", "-g", "-pthread", f"-I{include}", str(HERE / "cpp" / "query_pool.cpp"),
+                    str(CSRC / "query_pool.cpp"), "-o", str(out)], check=True)
+    return out
+
+
+def findings(exe, check):
+    """The lines a check prints, as dicts of its numbers."""
+    lines = subprocess.run([str(exe), check], check=True, capture_output=True, text=True, timeout=120).stdout.splitlines()
+    return [{k: int(v) for k, v in (w.split("=") for w in line.split()[1:])} for line in lines]
+
+
+def test_inputs_are_read_after_work_on_the_default_stream(exe):
+    found = findings(exe, "order")
+    assert [f["count"] for f in found] == [1, 1000, 300_007]
+    assert all(f["wrong"] == 0 for f in found), found
