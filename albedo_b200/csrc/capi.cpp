@@ -25,6 +25,7 @@
 #include <format>
 #include <memory>
 #include <new>
+#include <optional>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -208,7 +209,7 @@ BasicMaterialDesc basicFrom(const albedo_basic_material& m)
 
 namespace {
 
-// A committed scene's share in its device's ray-query buffers (runQueries).
+// A committed scene's share in its context's ray-query buffers (runQueries).
 class QueryShare {
 public:
     QueryShare() = default;
@@ -216,20 +217,25 @@ public:
     QueryShare& operator=(const QueryShare&) = delete;
     ~QueryShare()
     {
-        if (device_ >= 0) {
-            releaseQueryBuffers(device_);
+        if (context_) {
+            releaseQueryBuffers(*context_);
         }
     }
-    void hold(int device)
+    void hold()
     {
-        if (device_ < 0) {
-            retainQueryBuffers(device);
-            device_ = device;
+        if (!context_) {
+            try {
+                context_ = retainQueryBuffers();
+            } catch (const std::bad_alloc&) {
+                throw;
+            } catch (const std::exception& e) {
+                throw DeviceError{e.what()};
+            }
         }
     }
 
 private:
-    int device_{-1};
+    std::optional<std::uint64_t> context_;
 };
 
 } // namespace
@@ -316,9 +322,7 @@ struct albedo_scene {
         // has them; queries from host arrays run on streams that do not wait for
         // the default one.
         check(cudaStreamSynchronize(nullptr), "commit");
-        int device{0};
-        check(cudaGetDevice(&device), "cudaGetDevice");
-        query_share.hold(device);
+        query_share.hold();
         committed = true;
     }
 

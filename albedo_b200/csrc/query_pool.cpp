@@ -1,6 +1,8 @@
 // Worker buffers of host-array ray queries, and the chunk loop.
 #include "query_pool.hpp"
 
+#include <cuda.h>
+
 #include <algorithm>
 #include <array>
 #include <atomic>
@@ -40,6 +42,81 @@ void cudaCheck(cudaError_t e, const char* what)
     }
 }
 
+// The driver's context functions. The library links the runtime alone, which
+// hands out the driver's entry points.
+template <typename Function>
+Function driverFunction(const char* name)
+{
+    void* function{nullptr};
+    cudaDriverEntryPointQueryResult found{};
+    cudaCheck(cudaGetDriverEntryPointByVersion(name, &function, 12000, cudaEnableDefault, &found), name);
+    if (found != cudaDriverEntryPointSuccess || function == nullptr) {
+        throw std::runtime_error{std::format("{} is not in the driver", name)};
+    }
+    return reinterpret_cast<Function>(function);
+}
+
+struct Driver {
+    decltype(&cuCtxGetCurrent) current{driverFunction<decltype(&cuCtxGetCurrent)>("cuCtxGetCurrent")};
+    decltype(&cuCtxSetCurrent) makeCurrent{driverFunction<decltype(&cuCtxSetCurrent)>("cuCtxSetCurrent")};
+    decltype(&cuCtxGetId) id{driverFunction<decltype(&cuCtxGetId)>("cuCtxGetId")};
+    decltype(&cuCtxGetDevice) device{driverFunction<decltype(&cuCtxGetDevice)>("cuCtxGetDevice")};
+    decltype(&cuDevicePrimaryCtxGetState) primaryState{
+        driverFunction<decltype(&cuDevicePrimaryCtxGetState)>("cuDevicePrimaryCtxGetState")};
+    decltype(&cuDevicePrimaryCtxRetain) retainPrimary{
+        driverFunction<decltype(&cuDevicePrimaryCtxRetain)>("cuDevicePrimaryCtxRetain")};
+    decltype(&cuDevicePrimaryCtxRelease) releasePrimary{
+        driverFunction<decltype(&cuDevicePrimaryCtxRelease)>("cuDevicePrimaryCtxRelease")};
+};
+
+const Driver& driver()
+{
+    static const Driver functions;
+    return functions;
+}
+
+void driverCheck(CUresult e, const char* what)
+{
+    if (e != CUDA_SUCCESS) {
+        throw std::runtime_error{std::format("{}: driver error {}", what, static_cast<int>(e))};
+    }
+}
+
+// The context that is current in the calling thread: a scene's tables are there,
+// and so are a call's streams and buffers. It need not be its device's primary
+// one, which is what the runtime makes current in a thread that has none.
+struct CallContext {
+    CUcontext handle{nullptr};
+    std::uint64_t id{0}; // no other context of the process has it, before or after
+    bool primary{false};
+
+    static CallContext ofThisThread()
+    {
+        CallContext c;
+        driverCheck(driver().current(&c.handle), "current context");
+        if (c.handle == nullptr) {
+            // A thread without one: the runtime makes the primary context current.
+            cudaCheck(cudaFree(nullptr), "current context");
+            driverCheck(driver().current(&c.handle), "current context");
+        }
+        unsigned long long id{0};
+        driverCheck(driver().id(c.handle, &id), "context id");
+        c.id = id;
+        CUdevice device{};
+        unsigned int flags{0};
+        int active{0};
+        driverCheck(driver().device(&device), "context device");
+        driverCheck(driver().primaryState(device, &flags, &active), "primary context");
+        if (active != 0) {
+            CUcontext primary{nullptr};
+            driverCheck(driver().retainPrimary(&primary, device), "primary context");
+            c.primary = primary == c.handle;
+            driverCheck(driver().releasePrimary(device), "primary context");
+        }
+        return c;
+    }
+};
+
 // One worker's stream, pinned buffer and device buffer.
 struct Slot {
     cudaStream_t stream{nullptr};
@@ -72,9 +149,9 @@ struct Slot {
     }
 };
 
-// A device's slots: at most kMaxWorkers, made as they are needed; a worker that
+// A context's slots: at most kMaxWorkers, made as they are needed; a worker that
 // finds all of them in use waits for one.
-struct DevicePool {
+struct SlotPool {
     std::mutex mutex;
     std::condition_variable freed;
     std::vector<std::unique_ptr<Slot>> idle;
@@ -102,7 +179,7 @@ struct DevicePool {
         }
         return slot;
     }
-    // Puts a slot back; with no scene left on the device it is given up.
+    // Puts a slot back; with no scene left in the context it is given up.
     void give(std::unique_ptr<Slot> slot)
     {
         {
@@ -124,16 +201,19 @@ struct DevicePool {
     }
 };
 
-DevicePool& poolOf(int device)
+// The slots kept in a device's primary context. A context that a program made may
+// be destroyed while scenes of it are alive, and its streams with it: its slots
+// are a call's own (runQueries).
+SlotPool& poolOf(std::uint64_t context)
 {
     static std::mutex table_mutex;
     // Never destroyed: freeing device memory from a static destructor at exit
     // would run after the CUDA runtime has shut down.
-    static auto* table{new std::map<int, std::unique_ptr<DevicePool>>};
+    static auto* table{new std::map<std::uint64_t, std::unique_ptr<SlotPool>>};
     const std::lock_guard lock{table_mutex};
-    std::unique_ptr<DevicePool>& entry{(*table)[device]};
+    std::unique_ptr<SlotPool>& entry{(*table)[context]};
     if (!entry) {
-        entry = std::make_unique<DevicePool>();
+        entry = std::make_unique<SlotPool>();
     }
     return *entry;
 }
@@ -141,7 +221,7 @@ DevicePool& poolOf(int device)
 // A slot held by a worker.
 class HeldSlot {
 public:
-    explicit HeldSlot(DevicePool& pool) : pool_{pool}, slot_{pool.take()} {}
+    explicit HeldSlot(SlotPool& pool) : pool_{pool}, slot_{pool.take()} {}
     // A worker that failed may leave copies in flight that use the buffers.
     ~HeldSlot()
     {
@@ -153,7 +233,7 @@ public:
     Slot& operator*() const { return *slot_; }
 
 private:
-    DevicePool& pool_;
+    SlotPool& pool_;
     std::unique_ptr<Slot> slot_;
 };
 
@@ -222,9 +302,9 @@ void runQueries(std::int64_t count, std::span<const QueryInput> inputs, std::spa
     // memory takes asynchronous copies and kernels. The workers read and write the
     // arrays on the host, so that work has to be over first.
     cudaCheck(cudaStreamSynchronize(cudaStreamLegacy), "queries");
-    int device{0};
-    cudaCheck(cudaGetDevice(&device), "cudaGetDevice");
-    DevicePool& pool{poolOf(device)};
+    const CallContext context{CallContext::ofThisThread()};
+    SlotPool own;
+    SlotPool& pool{context.primary ? poolOf(context.id) : own};
     const std::int64_t share{(count + static_cast<std::int64_t>(kMaxWorkers) - 1) /
                              static_cast<std::int64_t>(kMaxWorkers)};
     const std::int64_t chunk{std::clamp(share, kMinChunk, kMaxChunk)};
@@ -245,7 +325,9 @@ void runQueries(std::int64_t count, std::span<const QueryInput> inputs, std::spa
         std::vector<std::jthread> threads;
         const auto guardedWork = [&](std::size_t k) {
             try {
-                cudaCheck(cudaSetDevice(device), "cudaSetDevice");
+                if (k > 0) {
+                    driverCheck(driver().makeCurrent(context.handle), "current context");
+                }
                 work();
             } catch (...) {
                 failed[k] = std::current_exception();
@@ -269,16 +351,21 @@ void runQueries(std::int64_t count, std::span<const QueryInput> inputs, std::spa
     }
 }
 
-void retainQueryBuffers(int device)
+std::optional<std::uint64_t> retainQueryBuffers()
 {
-    DevicePool& pool{poolOf(device)};
+    const CallContext context{CallContext::ofThisThread()};
+    if (!context.primary) {
+        return std::nullopt;
+    }
+    SlotPool& pool{poolOf(context.id)};
     const std::lock_guard lock{pool.mutex};
     ++pool.scenes;
+    return context.id;
 }
 
-void releaseQueryBuffers(int device)
+void releaseQueryBuffers(std::uint64_t context)
 {
-    DevicePool& pool{poolOf(device)};
+    SlotPool& pool{poolOf(context)};
     std::vector<std::unique_ptr<Slot>> given;
     {
         const std::lock_guard lock{pool.mutex};

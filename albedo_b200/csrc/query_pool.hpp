@@ -20,6 +20,7 @@
 #include <cstddef>
 #include <cstdint>
 #include <functional>
+#include <optional>
 #include <span>
 
 namespace albedo_b200 {
@@ -44,16 +45,18 @@ constexpr std::size_t kMaxQueryRayBytes{84};
 using QueryLaunch =
     std::function<cudaError_t(void* const* inputs, void* const* outputs, int count, cudaStream_t stream)>;
 
-// Runs `count` queries on the current device, after the work that the default
+// Runs `count` queries in the calling thread's current context, after the work that the default
 // stream held when the call was made, and returns when every result is in its
 // host array. Safe from several threads. Throws std::bad_alloc, or
 // std::runtime_error for any other CUDA failure.
 void runQueries(std::int64_t count, std::span<const QueryInput> inputs, std::span<const QueryOutput> outputs,
                 const QueryLaunch& launch);
 
-// A scene came to or left a device: the last one to leave gives the buffers
-// kept for that device's queries back.
-void retainQueryBuffers(int device);
-void releaseQueryBuffers(int device);
+// A scene came to the calling thread's current context, or left the context so
+// named: the last one to leave gives the buffers kept for its queries back. They
+// are kept in a device's primary context alone; elsewhere a call has its own, and
+// there is nothing to release.
+std::optional<std::uint64_t> retainQueryBuffers();
+void releaseQueryBuffers(std::uint64_t context);
 
 } // namespace albedo_b200

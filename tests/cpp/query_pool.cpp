@@ -1,11 +1,15 @@
 // Host checks of the ray-query workers (albedo_b200/csrc/query_pool.cpp) against a
 // stand-in for the CUDA runtime: device memory is host memory, work on the
 // workers' streams runs when it is enqueued, work on the default stream when
-// something waits for it.
+// something waits for it. Allocations and streams belong to the context that is
+// current in the thread that makes them.
 //
 // Arguments: the name of a check. Prints what it finds.
 #include "../../albedo_b200/csrc/query_pool.hpp"
 
+#include <cuda.h>
+
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -21,42 +25,146 @@ std::mutex mutex;
 // Work queued on the default stream.
 std::vector<std::function<void()>> default_stream;
 
+// Contexts 1 (the device's primary one, always active) and up; 0: none.
+thread_local std::uintptr_t current{0};
+std::atomic<int> used_elsewhere{0}; // pointers and streams used in another context than their own
+
+std::uintptr_t useCurrent()
+{
+    if (current == 0) {
+        current = 1;
+    }
+    return current;
+}
+
+// What is allocated, by address: its context and kind.
+struct Made {
+    std::uintptr_t context;
+    std::string kind;
+};
+std::map<const void*, Made> made;
+
+void* make(const char* kind, std::size_t bytes)
+{
+    void* p = std::malloc(bytes);
+    const std::lock_guard lock{mutex};
+    made[p] = {useCurrent(), kind};
+    return p;
+}
+cudaError_t unmake(const char* kind, void* p)
+{
+    if (p == nullptr) {
+        static_cast<void>(useCurrent());
+        return cudaSuccess;
+    }
+    const std::lock_guard lock{mutex};
+    const auto found = made.find(p);
+    if (found == made.end() || found->second.kind != kind) {
+        std::abort();
+    }
+    made.erase(found);
+    std::free(p);
+    return cudaSuccess;
+}
+// Counts a use of `p`, or of the allocation `p` points into, in another context.
+void use(const void* p)
+{
+    const std::lock_guard lock{mutex};
+    auto found = made.upper_bound(p);
+    if (found == made.begin() || (--found)->second.context != useCurrent()) {
+        ++used_elsewhere;
+    }
+}
+std::size_t alive()
+{
+    const std::lock_guard lock{mutex};
+    return made.size();
+}
+
+CUresult ctxGetCurrent(CUcontext* context)
+{
+    *context = reinterpret_cast<CUcontext>(current);
+    return CUDA_SUCCESS;
+}
+CUresult ctxSetCurrent(CUcontext context)
+{
+    current = reinterpret_cast<std::uintptr_t>(context);
+    return CUDA_SUCCESS;
+}
+CUresult ctxGetId(CUcontext context, unsigned long long* id)
+{
+    *id = 100 + reinterpret_cast<std::uintptr_t>(context);
+    return CUDA_SUCCESS;
+}
+CUresult ctxGetDevice(CUdevice* device)
+{
+    *device = 0;
+    return CUDA_SUCCESS;
+}
+CUresult primaryState(CUdevice, unsigned int*, int* active)
+{
+    *active = 1;
+    return CUDA_SUCCESS;
+}
+CUresult primaryRetain(CUcontext* context, CUdevice)
+{
+    *context = reinterpret_cast<CUcontext>(1);
+    return CUDA_SUCCESS;
+}
+CUresult primaryRelease(CUdevice) { return CUDA_SUCCESS; }
+
 } // namespace fake
 
 extern "C" {
 
+cudaError_t cudaGetDriverEntryPointByVersion(const char* name, void** function, unsigned int, unsigned long long,
+                                             cudaDriverEntryPointQueryResult* found)
+{
+    const std::map<std::string, void*> functions{
+        {"cuCtxGetCurrent", reinterpret_cast<void*>(fake::ctxGetCurrent)},
+        {"cuCtxSetCurrent", reinterpret_cast<void*>(fake::ctxSetCurrent)},
+        {"cuCtxGetId", reinterpret_cast<void*>(fake::ctxGetId)},
+        {"cuCtxGetDevice", reinterpret_cast<void*>(fake::ctxGetDevice)},
+        {"cuDevicePrimaryCtxGetState", reinterpret_cast<void*>(fake::primaryState)},
+        {"cuDevicePrimaryCtxRetain", reinterpret_cast<void*>(fake::primaryRetain)},
+        {"cuDevicePrimaryCtxRelease", reinterpret_cast<void*>(fake::primaryRelease)}};
+    const auto at = functions.find(name);
+    *function = at == functions.end() ? nullptr : at->second;
+    *found = *function == nullptr ? cudaDriverEntryPointSymbolNotFound : cudaDriverEntryPointSuccess;
+    return cudaSuccess;
+}
 cudaError_t cudaGetDevice(int* device)
 {
     *device = 0;
     return cudaSuccess;
 }
-cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaSetDevice(int)
+{
+    fake::current = 1;
+    return cudaSuccess;
+}
 const char* cudaGetErrorString(cudaError_t) { return "error"; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 
 cudaError_t cudaMalloc(void** p, size_t bytes)
 {
-    *p = std::malloc(bytes);
+    *p = fake::make("device", bytes);
     return cudaSuccess;
 }
-cudaError_t cudaFree(void* p)
+cudaError_t cudaFree(void* p) { return fake::unmake("device", p); }
+cudaError_t cudaMallocHost(void** p, size_t bytes)
 {
-    std::free(p);
+    *p = fake::make("pinned", bytes);
     return cudaSuccess;
 }
-cudaError_t cudaMallocHost(void** p, size_t bytes) { return cudaMalloc(p, bytes); }
-cudaError_t cudaFreeHost(void* p) { return cudaFree(p); }
+cudaError_t cudaFreeHost(void* p) { return fake::unmake("pinned", p); }
 
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* stream, unsigned int)
 {
-    *stream = reinterpret_cast<cudaStream_t>(std::malloc(1));
+    *stream = reinterpret_cast<cudaStream_t>(fake::make("stream", 1));
     return cudaSuccess;
 }
-cudaError_t cudaStreamDestroy(cudaStream_t stream)
-{
-    std::free(stream);
-    return cudaSuccess;
-}
+cudaError_t cudaStreamDestroy(cudaStream_t stream) { return fake::unmake("stream", stream); }
 cudaError_t cudaStreamSynchronize(cudaStream_t stream)
 {
     if (stream == nullptr || stream == cudaStreamLegacy) {
@@ -65,16 +173,23 @@ cudaError_t cudaStreamSynchronize(cudaStream_t stream)
             work();
         }
         fake::default_stream.clear();
+    } else {
+        fake::use(stream);
     }
     return cudaSuccess;
 }
-cudaError_t cudaMemcpyAsync(void* to, const void* from, size_t bytes, cudaMemcpyKind, cudaStream_t)
+cudaError_t cudaMemcpyAsync(void* to, const void* from, size_t bytes, cudaMemcpyKind, cudaStream_t stream)
 {
+    fake::use(to);
+    fake::use(from);
+    fake::use(stream);
     std::memcpy(to, from, bytes);
     return cudaSuccess;
 }
-cudaError_t cudaMemsetAsync(void* to, int value, size_t bytes, cudaStream_t)
+cudaError_t cudaMemsetAsync(void* to, int value, size_t bytes, cudaStream_t stream)
 {
+    fake::use(to);
+    fake::use(stream);
     std::memset(to, value, bytes);
     return cudaSuccess;
 }
@@ -86,8 +201,11 @@ namespace {
 using namespace albedo_b200;
 
 // A stand-in for a query: 2 v + 1 of each 4-byte input, nothing for negative ones.
-cudaError_t twicePlusOne(void* const* in, void* const* out, int count, cudaStream_t)
+cudaError_t twicePlusOne(void* const* in, void* const* out, int count, cudaStream_t stream)
 {
+    fake::use(in[0]);
+    fake::use(out[0]);
+    fake::use(stream);
     for (int i = 0; i < count; ++i) {
         const int v = static_cast<const int*>(in[0])[i];
         if (v >= 0) {
@@ -135,17 +253,54 @@ void order()
     }
 }
 
+// Calls in the primary context, in one of the program's own and in the primary
+// one again: everything is used where it was made, the caller's context stays, and
+// what is kept is kept in the primary one.
+void context()
+{
+    for (const std::uintptr_t own : {1, 7, 1}) {
+        fake::current = own;
+        const std::vector<int> in = numbers(300'007);
+        std::vector<int> out(in.size(), 5);
+        run(in, out);
+        std::printf("context own=%d after=%d wrong=%zu elsewhere=%d kept_elsewhere=%d\n", static_cast<int>(own),
+                    static_cast<int>(fake::current), wrongAnswers(in, out.data()), fake::used_elsewhere.load(),
+                    [] {
+                        int n = 0;
+                        for (const auto& [p, m] : fake::made) {
+                            n += m.context != 1 ? 1 : 0;
+                        }
+                        return n;
+                    }());
+    }
+}
+
+// With the last scene gone nothing is left; a scene of the program's own context
+// has no share.
+void scenes()
+{
+    const std::vector<int> in = numbers(300'007);
+    std::vector<int> out(in.size(), 5);
+    run(in, out);
+    const auto share = retainQueryBuffers();
+    releaseQueryBuffers(*share);
+    const std::size_t kept = fake::alive();
+    fake::current = 7;
+    std::printf("scenes kept=%d own_share=%d\n", kept > 0 ? 1 : 0, retainQueryBuffers() ? 1 : 0);
+}
+
 } // namespace
 
 int main(int argc, char** argv)
 {
-    const std::map<std::string, void (*)()> checks{{"order", order}};
+    const std::map<std::string, void (*)()> checks{{"order", order}, {"context", context}, {"scenes", scenes}};
     const auto check = checks.find(argc > 1 ? argv[1] : "");
     if (check == checks.end()) {
         return 2;
     }
-    retainQueryBuffers(0);
+    const auto share = retainQueryBuffers();
     check->second();
-    releaseQueryBuffers(0);
+    releaseQueryBuffers(*share);
+    std::printf("end left=%zu\n", fake::alive());
     return 0;
 }

@@ -26,8 +26,9 @@ def exe(tmp_path_factory):
 
 
 def findings(exe, check):
-    """The lines a check prints, as dicts of its numbers."""
+    """The lines a check prints, as dicts of its numbers; its last line says that nothing is left allocated."""
     lines = subprocess.run([str(exe), check], check=True, capture_output=True, text=True, timeout=120).stdout.splitlines()
+    assert lines.pop() == "end left=0"
     return [{k: int(v) for k, v in (w.split("=") for w in line.split()[1:])} for line in lines]
 
 
@@ -35,3 +36,14 @@ def test_inputs_are_read_after_work_on_the_default_stream(exe):
     found = findings(exe, "order")
     assert [f["count"] for f in found] == [1, 1000, 300_007]
     assert all(f["wrong"] == 0 for f in found), found
+
+
+def test_a_call_stays_in_its_threads_context(exe):
+    found = findings(exe, "context")
+    assert [f["own"] for f in found] == [1, 7, 1]
+    for f in found:
+        assert f["after"] == f["own"] and f["wrong"] == f["elsewhere"] == f["kept_elsewhere"] == 0, found
+
+
+def test_buffers_stay_while_a_scene_does(exe):
+    assert findings(exe, "scenes") == [{"kept": 1, "own_share": 0}]
