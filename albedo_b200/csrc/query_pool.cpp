@@ -30,7 +30,8 @@ constexpr std::int64_t kMinChunk{16384};
 constexpr std::int64_t kMaxChunk{32768};
 constexpr std::size_t kMaxWorkers{8};
 constexpr std::size_t kArrayAlign{256};
-constexpr std::size_t kSlotBytes{kMaxChunk * kMaxQueryRayBytes + 2 * kMaxQueryArrays * kArrayAlign};
+// Rays of the slot that serves a call where memory is short (90 KB of each).
+constexpr std::int64_t kFewRays{1024};
 
 void cudaCheck(cudaError_t e, const char* what)
 {
@@ -117,23 +118,39 @@ struct CallContext {
     }
 };
 
-// One worker's stream, pinned buffer and device buffer.
+// One worker's stream, pinned buffer and device buffer, for `rays` rays.
 struct Slot {
     cudaStream_t stream{nullptr};
     char* pinned{nullptr};
     char* device{nullptr};
+    std::int64_t rays{0};
 
     Slot() = default;
     Slot(const Slot&) = delete;
     Slot& operator=(const Slot&) = delete;
-    void allocate()
+    // Throws std::bad_alloc where there is no memory for it; the thread's CUDA
+    // error state is then clear again.
+    void allocate(std::int64_t count)
     {
-        cudaCheck(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "query stream");
+        const std::size_t bytes{static_cast<std::size_t>(count) * kMaxQueryRayBytes +
+                                2 * kMaxQueryArrays * kArrayAlign};
+        const auto need = [](cudaError_t e, const char* what) {
+            if (e == cudaErrorMemoryAllocation) {
+                static_cast<void>(cudaGetLastError());
+            }
+            cudaCheck(e, what);
+        };
+        if (stream == nullptr) {
+            need(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "query stream");
+        }
         void* p{nullptr};
-        cudaCheck(cudaMallocHost(&p, kSlotBytes), "query staging");
-        pinned = static_cast<char*>(p);
-        cudaCheck(cudaMalloc(&p, kSlotBytes), "query buffers");
+        if (pinned == nullptr) {
+            need(cudaMallocHost(&p, bytes), "query staging");
+            pinned = static_cast<char*>(p);
+        }
+        need(cudaMalloc(&p, bytes), "query buffers");
         device = static_cast<char*>(p);
+        rays = count;
     }
     ~Slot()
     {
@@ -149,8 +166,7 @@ struct Slot {
     }
 };
 
-// A context's slots: at most kMaxWorkers, made as they are needed; a worker that
-// finds all of them in use waits for one.
+// A context's slots: at most kMaxWorkers, made as they are needed.
 struct SlotPool {
     std::mutex mutex;
     std::condition_variable freed;
@@ -158,33 +174,64 @@ struct SlotPool {
     std::size_t made{0};
     int scenes{0};
 
+    // A slot for the caller of a query: waits for one while all are in use, and
+    // takes a small one where there is no memory for a whole one.
     std::unique_ptr<Slot> take()
     {
-        std::unique_lock lock{mutex};
-        freed.wait(lock, [&] { return !idle.empty() || made < kMaxWorkers; });
-        if (!idle.empty()) {
-            std::unique_ptr<Slot> slot{std::move(idle.back())};
-            idle.pop_back();
-            return slot;
+        {
+            std::unique_lock lock{mutex};
+            freed.wait(lock, [&] { return !idle.empty() || made < kMaxWorkers; });
+            if (!idle.empty()) {
+                return takeIdle();
+            }
+            ++made;
         }
-        ++made;
-        lock.unlock();
-        auto slot{std::make_unique<Slot>()};
         try {
-            slot->allocate();
+            std::unique_ptr<Slot> slot{std::make_unique<Slot>()};
+            try {
+                slot->allocate(kMaxChunk);
+            } catch (const std::bad_alloc&) {
+                slot->allocate(kFewRays);
+            }
+            return slot;
         } catch (...) {
-            slot.reset();
             drop();
             throw;
         }
-        return slot;
     }
-    // Puts a slot back; with no scene left in the context it is given up.
+    // A slot for a helper thread, or none: where all are in use or there is no
+    // memory for one, the other workers do its share.
+    std::unique_ptr<Slot> tryTake()
+    {
+        {
+            const std::lock_guard lock{mutex};
+            if (!idle.empty()) {
+                return takeIdle();
+            }
+            if (made == kMaxWorkers) {
+                return nullptr;
+            }
+            ++made;
+        }
+        try {
+            std::unique_ptr<Slot> slot{std::make_unique<Slot>()};
+            slot->allocate(kMaxChunk);
+            return slot;
+        } catch (const std::bad_alloc&) {
+            drop();
+            return nullptr;
+        } catch (...) {
+            drop();
+            throw;
+        }
+    }
+    // Puts a slot back; a small one, and any with no scene left in the context, is
+    // given up.
     void give(std::unique_ptr<Slot> slot)
     {
         {
             const std::lock_guard lock{mutex};
-            if (scenes > 0) {
+            if (scenes > 0 && slot->rays == kMaxChunk) {
                 idle.push_back(std::move(slot));
                 freed.notify_one();
                 return;
@@ -192,6 +239,14 @@ struct SlotPool {
         }
         slot.reset();
         drop();
+    }
+
+private:
+    std::unique_ptr<Slot> takeIdle()
+    {
+        std::unique_ptr<Slot> slot{std::move(idle.back())};
+        idle.pop_back();
+        return slot;
     }
     void drop()
     {
@@ -221,7 +276,7 @@ SlotPool& poolOf(std::uint64_t context)
 // A slot held by a worker.
 class HeldSlot {
 public:
-    explicit HeldSlot(SlotPool& pool) : pool_{pool}, slot_{pool.take()} {}
+    HeldSlot(SlotPool& pool, std::unique_ptr<Slot> slot) : pool_{pool}, slot_{std::move(slot)} {}
     // A worker that failed may leave copies in flight that use the buffers.
     ~HeldSlot()
     {
@@ -303,46 +358,59 @@ void runQueries(std::int64_t count, std::span<const QueryInput> inputs, std::spa
     // arrays on the host, so that work has to be over first.
     cudaCheck(cudaStreamSynchronize(cudaStreamLegacy), "queries");
     const CallContext context{CallContext::ofThisThread()};
-    SlotPool own;
-    SlotPool& pool{context.primary ? poolOf(context.id) : own};
+    SlotPool calls_own;
+    SlotPool& pool{context.primary ? poolOf(context.id) : calls_own};
     const std::int64_t share{(count + static_cast<std::int64_t>(kMaxWorkers) - 1) /
                              static_cast<std::int64_t>(kMaxWorkers)};
     const std::int64_t chunk{std::clamp(share, kMinChunk, kMaxChunk)};
     const std::int64_t chunks{(count + chunk - 1) / chunk};
     std::atomic<std::int64_t> next{0};
-    const auto work = [&] {
-        const HeldSlot slot{pool};
+    const auto work = [&](const Slot& slot) {
         for (std::int64_t c{next++}; c < chunks; c = next++) {
-            const std::int64_t first{c * chunk};
-            runChunk(*slot, static_cast<std::size_t>(first), static_cast<std::size_t>(std::min(chunk, count - first)),
-                     inputs, outputs, launch);
+            const std::int64_t end{std::min((c + 1) * chunk, count)};
+            for (std::int64_t first{c * chunk}; first < end; first += slot.rays) {
+                runChunk(slot, static_cast<std::size_t>(first),
+                         static_cast<std::size_t>(std::min(slot.rays, end - first)), inputs, outputs, launch);
+            }
         }
     };
     const std::size_t cores{std::max<std::size_t>(1, std::thread::hardware_concurrency())};
     const std::size_t workers{std::min({kMaxWorkers, cores, static_cast<std::size_t>(chunks)})};
     std::vector<std::exception_ptr> failed(workers);
-    {
-        std::vector<std::jthread> threads;
-        const auto guardedWork = [&](std::size_t k) {
-            try {
-                if (k > 0) {
-                    driverCheck(driver().makeCurrent(context.handle), "current context");
-                }
-                work();
-            } catch (...) {
-                failed[k] = std::current_exception();
-                next = chunks;
+    const auto guarded = [&](std::size_t k, const auto& body) {
+        try {
+            body();
+        } catch (...) {
+            failed[k] = std::current_exception();
+            next = chunks;
+        }
+    };
+    // The caller has a slot before there are helpers, so the call waits for no
+    // other slot and fails for want of memory only where nothing can run.
+    const HeldSlot own{pool, pool.take()};
+    const auto help = [&](std::size_t k) {
+        guarded(k, [&] {
+            if (next >= chunks) {
+                return;
             }
-        };
-        threads.reserve(workers - 1);
+            driverCheck(driver().makeCurrent(context.handle), "current context");
+            if (std::unique_ptr<Slot> slot{pool.tryTake()}) {
+                const HeldSlot held{pool, std::move(slot)};
+                work(*held);
+            }
+        });
+    };
+    {
+        std::vector<std::jthread> helpers;
+        helpers.reserve(workers - 1);
         try {
             for (std::size_t k{1}; k < workers; ++k) {
-                threads.emplace_back(guardedWork, k);
+                helpers.emplace_back(help, k);
             }
         } catch (const std::system_error&) {
             // Fewer threads than asked for: the ones that started share the chunks.
         }
-        guardedWork(0);
+        guarded(0, [&] { work(*own); });
     }
     for (const std::exception_ptr& e : failed) {
         if (e) {

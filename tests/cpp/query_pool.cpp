@@ -2,7 +2,7 @@
 // stand-in for the CUDA runtime: device memory is host memory, work on the
 // workers' streams runs when it is enqueued, work on the default stream when
 // something waits for it. Allocations and streams belong to the context that is
-// current in the thread that makes them.
+// current in the thread that makes them, and device memory may be short.
 //
 // Arguments: the name of a check. Prints what it finds.
 #include "../../albedo_b200/csrc/query_pool.hpp"
@@ -14,8 +14,10 @@
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <limits>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -37,18 +39,21 @@ std::uintptr_t useCurrent()
     return current;
 }
 
-// What is allocated, by address: its context and kind.
+// What is allocated, by address: its context, kind and size.
 struct Made {
     std::uintptr_t context;
     std::string kind;
+    std::size_t bytes;
 };
 std::map<const void*, Made> made;
+std::size_t device_limit{std::numeric_limits<std::size_t>::max()};
+thread_local cudaError_t last_error{cudaSuccess};
 
 void* make(const char* kind, std::size_t bytes)
 {
     void* p = std::malloc(bytes);
     const std::lock_guard lock{mutex};
-    made[p] = {useCurrent(), kind};
+    made[p] = {useCurrent(), kind, bytes};
     return p;
 }
 cudaError_t unmake(const char* kind, void* p)
@@ -144,10 +149,26 @@ cudaError_t cudaSetDevice(int)
     return cudaSuccess;
 }
 const char* cudaGetErrorString(cudaError_t) { return "error"; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError()
+{
+    const cudaError_t e = fake::last_error;
+    fake::last_error = cudaSuccess;
+    return e;
+}
 
 cudaError_t cudaMalloc(void** p, size_t bytes)
 {
+    std::size_t used = 0;
+    {
+        const std::lock_guard lock{fake::mutex};
+        for (const auto& [at, m] : fake::made) {
+            used += m.kind == "device" ? m.bytes : 0;
+        }
+    }
+    if (bytes > fake::device_limit || used > fake::device_limit - bytes) {
+        fake::last_error = cudaErrorMemoryAllocation;
+        return cudaErrorMemoryAllocation;
+    }
     *p = fake::make("device", bytes);
     return cudaSuccess;
 }
@@ -212,7 +233,7 @@ cudaError_t twicePlusOne(void* const* in, void* const* out, int count, cudaStrea
             static_cast<int*>(out[0])[i] = 2 * v + 1;
         }
     }
-    return cudaSuccess;
+    return cudaGetLastError(); // as a launch reports what went wrong before it
 }
 
 std::vector<int> numbers(std::size_t count)
@@ -289,11 +310,34 @@ void scenes()
     std::printf("scenes kept=%d own_share=%d\n", kept > 0 ? 1 : 0, retainQueryBuffers() ? 1 : 0);
 }
 
+// Device memory for nothing, for a small slot, for one slot and for three of those
+// a call would use, and without a limit; ten calls each.
+void memory()
+{
+    const std::vector<int> in = numbers(300'007);
+    for (const std::size_t limit : {std::size_t{0}, std::size_t{100'000}, std::size_t{3'000'000},
+                                    std::size_t{9'000'000}, std::numeric_limits<std::size_t>::max()}) {
+        fake::device_limit = limit;
+        for (int k = 0; k < 10; ++k) {
+            std::vector<int> out(in.size(), 5);
+            bool refused = false;
+            try {
+                run(in, out);
+            } catch (const std::bad_alloc&) {
+                refused = true;
+            }
+            std::printf("memory limit=%zu refused=%d wrong=%zu error=%d\n", limit, refused ? 1 : 0,
+                        refused ? std::size_t{0} : wrongAnswers(in, out.data()), static_cast<int>(cudaGetLastError()));
+        }
+    }
+}
+
 } // namespace
 
 int main(int argc, char** argv)
 {
-    const std::map<std::string, void (*)()> checks{{"order", order}, {"context", context}, {"scenes", scenes}};
+    const std::map<std::string, void (*)()> checks{{"order", order}, {"context", context}, {"scenes", scenes},
+                                                      {"memory", memory}};
     const auto check = checks.find(argc > 1 ? argv[1] : "");
     if (check == checks.end()) {
         return 2;

@@ -47,3 +47,10 @@ def test_a_call_stays_in_its_threads_context(exe):
 
 def test_buffers_stay_while_a_scene_does(exe):
     assert findings(exe, "scenes") == [{"kept": 1, "own_share": 0}]
+
+
+def test_a_call_runs_with_the_buffers_there_is_memory_for(exe):
+    found = findings(exe, "memory")
+    assert len(found) == 50
+    for f in found:
+        assert f["refused"] == (1 if f["limit"] == 0 else 0) and f["wrong"] == f["error"] == 0, f
