@@ -333,6 +333,61 @@ void runChunk(const Slot& slot, std::size_t first, std::size_t n, std::span<cons
 
 } // namespace
 
+namespace {
+
+// Whether an output of the call shares memory with another of its arrays.
+bool arraysOverlap(std::size_t count, std::span<const QueryInput> inputs, std::span<const QueryOutput> outputs)
+{
+    const auto shared = [&](const QueryOutput& a, const void* host, std::size_t ray_bytes) {
+        const auto at{reinterpret_cast<std::uintptr_t>(a.host)};
+        const auto other{reinterpret_cast<std::uintptr_t>(host)};
+        return a.host != nullptr && host != nullptr && at < other + count * ray_bytes &&
+               other < at + count * a.ray_bytes;
+    };
+    for (std::size_t i{0}; i < outputs.size(); ++i) {
+        for (const QueryInput& in : inputs) {
+            if (shared(outputs[i], in.host, in.ray_bytes)) {
+                return true;
+            }
+        }
+        for (std::size_t k{i + 1}; k < outputs.size(); ++k) {
+            if (shared(outputs[i], outputs[k].host, outputs[k].ray_bytes)) {
+                return true;
+            }
+        }
+    }
+    return false;
+}
+
+// A call whose outputs lie over its inputs or each other reads every input before
+// it writes a result and writes its outputs whole, one after the other; its chunks,
+// which run beside each other, work on copies.
+void runOnCopies(std::int64_t count, std::span<const QueryInput> inputs, std::span<const QueryOutput> outputs,
+                 const QueryLaunch& launch)
+{
+    const auto n{static_cast<std::size_t>(count)};
+    std::vector<std::vector<char>> memory;
+    std::vector<QueryInput> in{inputs.begin(), inputs.end()};
+    for (QueryInput& i : in) {
+        const char* const host{static_cast<const char*>(i.host)};
+        i.host = memory.emplace_back(host, host + n * i.ray_bytes).data();
+    }
+    std::vector<QueryOutput> out{outputs.begin(), outputs.end()};
+    for (QueryOutput& o : out) {
+        if (o.host != nullptr) {
+            o.host = memory.emplace_back(n * o.ray_bytes).data();
+        }
+    }
+    runQueries(count, in, out, launch);
+    for (std::size_t i{0}; i < outputs.size(); ++i) {
+        if (outputs[i].host != nullptr) {
+            std::memcpy(outputs[i].host, out[i].host, n * outputs[i].ray_bytes);
+        }
+    }
+}
+
+} // namespace
+
 void runQueries(std::int64_t count, std::span<const QueryInput> inputs, std::span<const QueryOutput> outputs,
                 const QueryLaunch& launch)
 {
@@ -357,6 +412,9 @@ void runQueries(std::int64_t count, std::span<const QueryInput> inputs, std::spa
     // memory takes asynchronous copies and kernels. The workers read and write the
     // arrays on the host, so that work has to be over first.
     cudaCheck(cudaStreamSynchronize(cudaStreamLegacy), "queries");
+    if (arraysOverlap(static_cast<std::size_t>(count), inputs, outputs)) {
+        return runOnCopies(count, inputs, outputs, launch);
+    }
     const CallContext context{CallContext::ofThisThread()};
     SlotPool calls_own;
     SlotPool& pool{context.primary ? poolOf(context.id) : calls_own};

@@ -9,6 +9,7 @@
 
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -332,12 +333,51 @@ void memory()
     }
 }
 
+// Outputs over the inputs, in place and shifted either way, and two outputs over each other.
+void overlap()
+{
+    for (const std::size_t count : {std::size_t{1}, std::size_t{20'000}, std::size_t{300'007}}) {
+        const std::vector<int> in = numbers(count);
+        for (const std::size_t before : {std::size_t{0}, std::size_t{1}, count / 2}) {
+            for (const std::size_t behind : {std::size_t{0}, std::size_t{1}, count / 2}) {
+                std::vector<int> both(count + before + behind);
+                std::copy(in.begin(), in.end(), both.begin() + static_cast<std::ptrdiff_t>(before));
+                int* const results = both.data() + behind;
+                const QueryInput inputs[]{{both.data() + before, sizeof(int)}};
+                const QueryOutput outputs[]{{results, sizeof(int)}};
+                runQueries(static_cast<std::int64_t>(count), inputs, outputs, twicePlusOne);
+                std::printf("overlap count=%zu wrong=%zu\n", count, wrongAnswers(in, results));
+            }
+        }
+        // The second output, 12 bytes a ray, ends up whole, the first where it reaches beyond it.
+        std::vector<int> both(4 * count);
+        const QueryInput inputs[]{{in.data(), sizeof(int)}};
+        const QueryOutput outputs[]{{both.data() + 3 * count - count / 2, sizeof(int)}, {both.data(), 3 * sizeof(int)}};
+        runQueries(static_cast<std::int64_t>(count), inputs, outputs,
+                   [](void* const* i, void* const* o, int n, cudaStream_t stream) {
+                       for (int k = 0; k < 3 * n; ++k) {
+                           static_cast<int*>(o[1])[k] = -7;
+                       }
+                       return twicePlusOne(i, o, n, stream);
+                   });
+        std::size_t wrong = 0;
+        for (std::size_t k = 0; k < 3 * count; ++k) {
+            wrong += both[k] != -7 ? 1 : 0;
+        }
+        for (std::size_t k = count / 2; k < count; ++k) {
+            const int v = in[k];
+            wrong += both[3 * count - count / 2 + k] != (v < 0 ? 0 : 2 * v + 1) ? 1 : 0;
+        }
+        std::printf("overlap count=%zu wrong=%zu\n", count, wrong);
+    }
+}
+
 } // namespace
 
 int main(int argc, char** argv)
 {
     const std::map<std::string, void (*)()> checks{{"order", order}, {"context", context}, {"scenes", scenes},
-                                                      {"memory", memory}};
+                                                      {"memory", memory}, {"overlap", overlap}};
     const auto check = checks.find(argc > 1 ? argv[1] : "");
     if (check == checks.end()) {
         return 2;

@@ -54,3 +54,8 @@ def test_a_call_runs_with_the_buffers_there_is_memory_for(exe):
     assert len(found) == 50
     for f in found:
         assert f["refused"] == (1 if f["limit"] == 0 else 0) and f["wrong"] == f["error"] == 0, f
+
+
+def test_outputs_over_other_arrays_are_written_after_they_are_read(exe):
+    found = findings(exe, "overlap")
+    assert len(found) == 30 and all(f["wrong"] == 0 for f in found), found
