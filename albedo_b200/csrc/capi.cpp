@@ -1663,11 +1663,10 @@ int albedo_scene_check(const albedo_scene* scene)
 
 namespace {
 
-// Throws for an array in device memory and, when `needed`, for a null one.
-void requireHostArray(const void* array, bool needed)
+// Throws for an array in device memory.
+void requireHostArray(const void* array)
 {
     if (array == nullptr) {
-        check(needed ? cudaErrorInvalidValue : cudaSuccess, "upload");
         return;
     }
     cudaPointerAttributes at{};
@@ -1680,12 +1679,18 @@ void hostQueries(int64_t count, std::span<const QueryInput> inputs, std::span<co
                  const QueryLaunch& launch)
 {
     // The workers read and write the arrays with the host's own copies: what those
-    // cannot touch is refused, as a copy by the driver would have.
-    for (const QueryInput& in : inputs) {
-        requireHostArray(in.host, count > 0);
-    }
-    for (const QueryOutput& out : outputs) {
-        requireHostArray(out.host, false);
+    // cannot touch is refused, as a copy by the driver would have. Arrays that a
+    // call does not use (no rays, no geometry asked for) may be anything.
+    if (count > 0) {
+        for (const QueryInput& in : inputs) {
+            check(in.host == nullptr ? cudaErrorInvalidValue : cudaSuccess, "upload");
+            requireHostArray(in.host);
+        }
+        for (const QueryOutput& out : outputs) {
+            if (out.ray_bytes > 0) {
+                requireHostArray(out.host);
+            }
+        }
     }
     try {
         runQueries(count, inputs, outputs, launch);

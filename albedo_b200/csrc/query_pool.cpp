@@ -331,10 +331,6 @@ void runChunk(const Slot& slot, std::size_t first, std::size_t n, std::span<cons
     }
 }
 
-} // namespace
-
-namespace {
-
 // Whether an output of the call shares memory with another of its arrays.
 bool arraysOverlap(std::size_t count, std::span<const QueryInput> inputs, std::span<const QueryOutput> outputs)
 {
