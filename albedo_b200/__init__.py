@@ -503,8 +503,9 @@ class Server:
             pass
 
 
-def wavefront_configure(slots: int = 1 << 20, blocks_per_sm: int = 8, iterations_per_graph: int = 4) -> None:
-    """Shape of the wavefront engine: path slots, queue-kernel blocks per SM, iterations per graph."""
+def wavefront_configure(slots: int = 1 << 20, blocks_per_sm: int = 4, iterations_per_graph: int = 4) -> None:
+    """Shape of the wavefront engine: path slots, queue-kernel blocks per SM, iterations per graph.
+    The defaults are those of an engine that has not been configured."""
     _raise(library().albedo_wavefront_configure(slots, blocks_per_sm, iterations_per_graph))
 
 

@@ -310,8 +310,9 @@ int albedo_server_routes(const albedo_server* server, int64_t* out_batched, int6
 int albedo_server_release_scene(albedo_server* server, const albedo_scene* scene);
 void albedo_server_destroy(albedo_server* server);
 /* Wavefront engine shape: path slots, blocks per SM of the queue kernels, and
- * iterations per captured CUDA graph; the traversal kernels' blocks per SM and
- * fetch batch return to their defaults (as many as fit, 32). */
+ * iterations per captured CUDA graph (by default 2^20, 4 and 4); the traversal
+ * kernels' blocks per SM and fetch batch return to their defaults (as many as fit,
+ * 32). */
 int albedo_wavefront_configure(int32_t slot_count, int32_t blocks_per_sm, int32_t iterations_per_graph);
 /* Autotuner. No counterpart in the reference (a CPU renderer with no launch
  * shapes). Candidate launch shapes are timed with CUDA events on the caller's
