@@ -129,7 +129,7 @@ cudaError_t renderNoAlloc(const WfJob& job, int stack, int blocks, unsigned int*
         return e;
     }
     // Rays in fetches of 32, one traversal step a turn (the engine's default).
-    const WfLaunch launch{blocks, 128, stack, per_sm * sms, 32, 1};
+    const WfLaunch launch{blocks, 128, stack, per_sm * sms, 32, 1, 0, shadeBlocks(blocks, sms)};
     // A slot finishes its pixel within n^2 (max_depth + 2) iterations: the
     // total iteration bound (computed in 64 bits; max_depth may be near INT_MAX).
     const unsigned long long bound = static_cast<unsigned long long>(job.samples_per_axis) * job.samples_per_axis *

@@ -817,12 +817,7 @@ cudaError_t wfIteration(const WfJob* jobs, const WfBuffers& b, const WfLaunch& l
     const int fetch = launch.fetch_batch > 0 ? launch.fetch_batch : 32;
     // The persistent traversal kernels keep 4-byte stack entries (references only).
     const auto smemFor = [](int entries) { return static_cast<std::size_t>(entries) * 128 * sizeof(unsigned); };
-    // The four shade kernels run beside each other, and each leaves room for the
-    // others at three blocks per SM of the default four: trefoil frame at 16
-    // samples 46.8 ms against 49.3 at four and 49.7 at eight, 16-job batch 102.4 /
-    // 103.4 / 104.1, sphere room 8.2 / 8.3 / 8.5; two are slower again (47.7, 103.3,
-    // 8.3).
-    const int sg = g >= 4 ? g / 4 * 3 : g;
+    const int sg = launch.shade_blocks;
     regenKernel<<<g, 128, 0, stream>>>(jobs, b);
     const bool binned = launch.ray_sort != 0 && b.binned != nullptr;
     if (binned) {

@@ -146,7 +146,24 @@ struct WfLaunch {
     int trace_loop;   // traversal turn shape of the persistent kernels (TraceLoop)
     int ray_sort;     // 1: the extend queue is binned by ray coherence before the extend kernel; 2: the shadow
                       // queue too
+    int shade_blocks; // grid of each shade kernel
 };
+
+// Grid of each shade kernel where the queue kernels have `blocks` blocks. The four
+// run beside each other, and at three quarters of the default four blocks per SM
+// each leaves room for the others: trefoil frame at 16 samples 46.8 ms against 49.3
+// at four and 49.7 at eight, 16-job batch 102.4 / 103.4 / 104.1, sphere room 8.2 /
+// 8.3 / 8.5. Two per SM are slower again (47.7, 103.3, 8.3), so a grid of three and
+// fewer is not cut.
+constexpr int shadeBlocks(int blocks, int sms)
+{
+    const int least = blocks < 3 * sms ? blocks : 3 * sms;
+    const int share = blocks / 4 * 3;
+    return share > least ? share : least;
+}
+static_assert(shadeBlocks(148, 148) == 148 && shadeBlocks(2 * 148, 148) == 2 * 148);
+static_assert(shadeBlocks(3 * 148, 148) == 3 * 148 && shadeBlocks(4 * 148, 148) == 3 * 148);
+static_assert(shadeBlocks(8 * 148, 148) == 6 * 148 && shadeBlocks(16 * 148, 148) == 12 * 148);
 
 // Opts the traversal kernels into `stack` entries of dynamic shared memory; call
 // before capturing iterations into a graph.

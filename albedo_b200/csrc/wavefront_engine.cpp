@@ -133,7 +133,8 @@ void WavefrontEngine::open(int stack, unsigned int* error_flag)
         trace_per_sm = std::min(trace_per_sm, shape_.trace_blocks_per_sm);
     }
     const WfLaunch launch{sm_count_ * shape_.blocks_per_sm, 128, stack, sm_count_ * trace_per_sm, shape_.fetch_batch,
-                          shape_.trace_loop, shape_.ray_sort};
+                          shape_.trace_loop, shape_.ray_sort,
+                          shadeBlocks(sm_count_ * shape_.blocks_per_sm, sm_count_)};
     cudaGraph_t graph{nullptr};
     cudaCheck(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "capture begin");
     cudaError_t captured{cudaSuccess};

@@ -15,7 +15,7 @@ namespace albedo_b200 {
 
 // Launch shape of the wavefront iteration (the autotuner's knobs).
 struct WfShape {
-    int blocks_per_sm{4};         // queue kernels: blocks per SM (regenerate; the shade kernels take 3/4 of it)
+    int blocks_per_sm{4};         // queue kernels: blocks per SM (the shade kernels take shadeBlocks of it)
     int iterations_per_graph{4};  // iterations captured in one CUDA graph
     int trace_blocks_per_sm{0};   // persistent traversal kernels: blocks per SM, 0 = as many as fit
     int fetch_batch{32};          // queue entries a traversal warp claims at once

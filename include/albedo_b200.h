@@ -327,7 +327,9 @@ typedef struct albedo_tuning {
                                      the path estimator keeps each path's state in shared memory;
                                      a scene without a shape of its own takes 3, or 4 for large
                                      images, and reads 3 here);
-                                     wavefront: blocks per SM of the queue kernels */
+                                     wavefront: blocks per SM of the queue kernels; the four shade
+                                     kernels, which run beside each other, take three quarters of
+                                     it each, or 3 where that is less */
     int32_t trace_blocks_per_sm;  /* wavefront: persistent traversal blocks per SM */
     int32_t fetch_batch;          /* wavefront: queue entries a traversal warp claims at once */
     int32_t iterations_per_graph; /* wavefront: iterations per captured CUDA graph */
