@@ -25,7 +25,6 @@
 #include <format>
 #include <memory>
 #include <new>
-#include <optional>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -215,27 +214,24 @@ public:
     QueryShare() = default;
     QueryShare(const QueryShare&) = delete;
     QueryShare& operator=(const QueryShare&) = delete;
-    ~QueryShare()
-    {
-        if (context_) {
-            releaseQueryBuffers(*context_);
-        }
-    }
+    ~QueryShare() { releaseQueryBuffers(slots_); }
     void hold()
     {
-        if (!context_) {
-            try {
-                context_ = retainQueryBuffers();
-            } catch (const std::bad_alloc&) {
-                throw;
-            } catch (const std::exception& e) {
-                throw DeviceError{e.what()};
-            }
+        if (slots_ != nullptr) {
+            return;
+        }
+        try {
+            slots_ = retainQueryBuffers();
+        } catch (const std::bad_alloc&) {
+            throw;
+        } catch (const std::exception& e) {
+            throw DeviceError{e.what()};
         }
     }
+    SlotPool* slots() const { return slots_; }
 
 private:
-    std::optional<std::uint64_t> context_;
+    SlotPool* slots_{nullptr};
 };
 
 } // namespace
@@ -1675,8 +1671,8 @@ void requireHostArray(const void* array)
 }
 
 // runQueries with its CUDA failures as device errors.
-void hostQueries(int64_t count, std::span<const QueryInput> inputs, std::span<const QueryOutput> outputs,
-                 const QueryLaunch& launch)
+void hostQueries(const albedo_scene& scene, int64_t count, std::span<const QueryInput> inputs,
+                 std::span<const QueryOutput> outputs, const QueryLaunch& launch)
 {
     // The workers read and write the arrays with the host's own copies: what those
     // cannot touch is refused, as a copy by the driver would have. Arrays that a
@@ -1693,7 +1689,7 @@ void hostQueries(int64_t count, std::span<const QueryInput> inputs, std::span<co
         }
     }
     try {
-        runQueries(count, inputs, outputs, launch);
+        runQueries(scene.query_share.slots(), count, inputs, outputs, launch);
     } catch (const std::bad_alloc&) {
         throw;
     } catch (const std::exception& e) {
@@ -1713,7 +1709,7 @@ void closestHits(const albedo_scene& scene, const float* rays, int64_t count, fl
     const QueryOutput outputs[]{{hit, sizeof(int)},       {t, sizeof(float)}, {object, sizeof(int)},
                                 {triangle, sizeof(int)},  {point, three},     {normal, three},
                                 {shading_normal, three},  {front, geometry ? sizeof(int) : 0}};
-    hostQueries(count, inputs, outputs, [&](void* const* in, void* const* out, int n, cudaStream_t stream) {
+    hostQueries(scene, count, inputs, outputs, [&](void* const* in, void* const* out, int n, cudaStream_t stream) {
         const auto floats = [&](int i) { return static_cast<float*>(out[i]); };
         const auto ints = [&](int i) { return static_cast<int*>(out[i]); };
         const TraceOutputs to{ints(0),
@@ -1749,7 +1745,7 @@ int albedo_occluded_host(const albedo_scene* scene, const float* rays, const flo
         scene->requireCommitted();
         const QueryInput inputs[]{{rays, 6 * sizeof(float)}, {t_max, sizeof(float)}};
         const QueryOutput outputs[]{{occluded, sizeof(int)}};
-        hostQueries(count, inputs, outputs, [&](void* const* in, void* const* out, int n, cudaStream_t stream) {
+        hostQueries(*scene, count, inputs, outputs, [&](void* const* in, void* const* out, int n, cudaStream_t stream) {
             return launchOccluded(scene->dev, static_cast<const float*>(in[0]), static_cast<const float*>(in[1]), n,
                                   static_cast<int*>(out[0]), scene->error_flag.as<unsigned int>(),
                                   scene->stack_capacity, stream);

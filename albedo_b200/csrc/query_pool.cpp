@@ -86,37 +86,32 @@ void driverCheck(CUresult e, const char* what)
 // The context that is current in the calling thread: a scene's tables are there,
 // and so are a call's streams and buffers. It need not be its device's primary
 // one, which is what the runtime makes current in a thread that has none.
-struct CallContext {
-    CUcontext handle{nullptr};
-    std::uint64_t id{0}; // no other context of the process has it, before or after
-    bool primary{false};
-
-    static CallContext ofThisThread()
-    {
-        CallContext c;
-        driverCheck(driver().current(&c.handle), "current context");
-        if (c.handle == nullptr) {
-            // A thread without one: the runtime makes the primary context current.
-            cudaCheck(cudaFree(nullptr), "current context");
-            driverCheck(driver().current(&c.handle), "current context");
-        }
-        unsigned long long id{0};
-        driverCheck(driver().id(c.handle, &id), "context id");
-        c.id = id;
-        CUdevice device{};
-        unsigned int flags{0};
-        int active{0};
-        driverCheck(driver().device(&device), "context device");
-        driverCheck(driver().primaryState(device, &flags, &active), "primary context");
-        if (active != 0) {
-            CUcontext primary{nullptr};
-            driverCheck(driver().retainPrimary(&primary, device), "primary context");
-            c.primary = primary == c.handle;
-            driverCheck(driver().releasePrimary(device), "primary context");
-        }
-        return c;
+CUcontext currentContext()
+{
+    CUcontext context{nullptr};
+    driverCheck(driver().current(&context), "current context");
+    if (context == nullptr) {
+        cudaCheck(cudaFree(nullptr), "current context");
+        driverCheck(driver().current(&context), "current context");
     }
-};
+    return context;
+}
+
+bool isPrimary(CUcontext context)
+{
+    CUdevice device{};
+    unsigned int flags{0};
+    int active{0};
+    driverCheck(driver().device(&device), "context device");
+    driverCheck(driver().primaryState(device, &flags, &active), "primary context");
+    if (active == 0) {
+        return false;
+    }
+    CUcontext primary{nullptr};
+    driverCheck(driver().retainPrimary(&primary, device), "primary context");
+    driverCheck(driver().releasePrimary(device), "primary context");
+    return primary == context;
+}
 
 // One worker's stream, pinned buffer and device buffer, for `rays` rays.
 struct Slot {
@@ -166,7 +161,8 @@ struct Slot {
     }
 };
 
-// A context's slots: at most kMaxWorkers, made as they are needed.
+} // namespace
+
 struct SlotPool {
     std::mutex mutex;
     std::condition_variable freed;
@@ -256,10 +252,11 @@ private:
     }
 };
 
-// The slots kept in a device's primary context. A context that a program made may
-// be destroyed while scenes of it are alive, and its streams with it: its slots
-// are a call's own (runQueries).
-SlotPool& poolOf(std::uint64_t context)
+namespace {
+
+// The slots kept in a primary context, by the driver's id for it, which no other
+// context of the process has, before or after.
+SlotPool& keptSlots(std::uint64_t context)
 {
     static std::mutex table_mutex;
     // Never destroyed: freeing device memory from a static destructor at exit
@@ -358,7 +355,7 @@ bool arraysOverlap(std::size_t count, std::span<const QueryInput> inputs, std::s
 // A call whose outputs lie over its inputs or each other reads every input before
 // it writes a result and writes its outputs whole, one after the other; its chunks,
 // which run beside each other, work on copies.
-void runOnCopies(std::int64_t count, std::span<const QueryInput> inputs, std::span<const QueryOutput> outputs,
+void runOnCopies(SlotPool* kept, std::int64_t count, std::span<const QueryInput> inputs, std::span<const QueryOutput> outputs,
                  const QueryLaunch& launch)
 {
     const auto n{static_cast<std::size_t>(count)};
@@ -374,7 +371,7 @@ void runOnCopies(std::int64_t count, std::span<const QueryInput> inputs, std::sp
             o.host = memory.emplace_back(n * o.ray_bytes).data();
         }
     }
-    runQueries(count, in, out, launch);
+    runQueries(kept, count, in, out, launch);
     for (std::size_t i{0}; i < outputs.size(); ++i) {
         if (outputs[i].host != nullptr) {
             std::memcpy(outputs[i].host, out[i].host, n * outputs[i].ray_bytes);
@@ -384,8 +381,8 @@ void runOnCopies(std::int64_t count, std::span<const QueryInput> inputs, std::sp
 
 } // namespace
 
-void runQueries(std::int64_t count, std::span<const QueryInput> inputs, std::span<const QueryOutput> outputs,
-                const QueryLaunch& launch)
+void runQueries(SlotPool* kept, std::int64_t count, std::span<const QueryInput> inputs,
+                std::span<const QueryOutput> outputs, const QueryLaunch& launch)
 {
     if (count < 0) {
         throw std::bad_alloc{};
@@ -409,11 +406,10 @@ void runQueries(std::int64_t count, std::span<const QueryInput> inputs, std::spa
     // arrays on the host, so that work has to be over first.
     cudaCheck(cudaStreamSynchronize(cudaStreamLegacy), "queries");
     if (arraysOverlap(static_cast<std::size_t>(count), inputs, outputs)) {
-        return runOnCopies(count, inputs, outputs, launch);
+        return runOnCopies(kept, count, inputs, outputs, launch);
     }
-    const CallContext context{CallContext::ofThisThread()};
     SlotPool calls_own;
-    SlotPool& pool{context.primary ? poolOf(context.id) : calls_own};
+    SlotPool& pool{kept != nullptr ? *kept : calls_own};
     const std::int64_t share{(count + static_cast<std::int64_t>(kMaxWorkers) - 1) /
                              static_cast<std::int64_t>(kMaxWorkers)};
     const std::int64_t chunk{std::clamp(share, kMinChunk, kMaxChunk)};
@@ -430,6 +426,7 @@ void runQueries(std::int64_t count, std::span<const QueryInput> inputs, std::spa
     };
     const std::size_t cores{std::max<std::size_t>(1, std::thread::hardware_concurrency())};
     const std::size_t workers{std::min({kMaxWorkers, cores, static_cast<std::size_t>(chunks)})};
+    const CUcontext context{workers > 1 ? currentContext() : nullptr};
     std::vector<std::exception_ptr> failed(workers);
     const auto guarded = [&](std::size_t k, const auto& body) {
         try {
@@ -447,7 +444,7 @@ void runQueries(std::int64_t count, std::span<const QueryInput> inputs, std::spa
             if (next >= chunks) {
                 return;
             }
-            driverCheck(driver().makeCurrent(context.handle), "current context");
+            driverCheck(driver().makeCurrent(context), "current context");
             if (std::unique_ptr<Slot> slot{pool.tryTake()}) {
                 const HeldSlot held{pool, std::move(slot)};
                 work(*held);
@@ -473,30 +470,34 @@ void runQueries(std::int64_t count, std::span<const QueryInput> inputs, std::spa
     }
 }
 
-std::optional<std::uint64_t> retainQueryBuffers()
+SlotPool* retainQueryBuffers()
 {
-    const CallContext context{CallContext::ofThisThread()};
-    if (!context.primary) {
-        return std::nullopt;
+    const CUcontext context{currentContext()};
+    if (!isPrimary(context)) {
+        return nullptr;
     }
-    SlotPool& pool{poolOf(context.id)};
+    unsigned long long id{0};
+    driverCheck(driver().id(context, &id), "context id");
+    SlotPool& pool{keptSlots(id)};
     const std::lock_guard lock{pool.mutex};
     ++pool.scenes;
-    return context.id;
+    return &pool;
 }
 
-void releaseQueryBuffers(std::uint64_t context)
+void releaseQueryBuffers(SlotPool* kept)
 {
-    SlotPool& pool{poolOf(context)};
+    if (kept == nullptr) {
+        return;
+    }
     std::vector<std::unique_ptr<Slot>> given;
     {
-        const std::lock_guard lock{pool.mutex};
-        if (--pool.scenes > 0) {
+        const std::lock_guard lock{kept->mutex};
+        if (--kept->scenes > 0) {
             return;
         }
-        given.swap(pool.idle);
-        pool.made -= given.size();
-        pool.freed.notify_all();
+        given.swap(kept->idle);
+        kept->made -= given.size();
+        kept->freed.notify_all();
     }
 }
 

@@ -20,7 +20,6 @@
 #include <cstddef>
 #include <cstdint>
 #include <functional>
-#include <optional>
 #include <span>
 
 namespace albedo_b200 {
@@ -45,18 +44,22 @@ constexpr std::size_t kMaxQueryRayBytes{84};
 using QueryLaunch =
     std::function<cudaError_t(void* const* inputs, void* const* outputs, int count, cudaStream_t stream)>;
 
-// Runs `count` queries in the calling thread's current context, after the work that the default
-// stream held when the call was made, and returns when every result is in its
-// host array. Safe from several threads. Throws std::bad_alloc, or
-// std::runtime_error for any other CUDA failure.
-void runQueries(std::int64_t count, std::span<const QueryInput> inputs, std::span<const QueryOutput> outputs,
-                const QueryLaunch& launch);
+// A context's slots (a worker's stream and buffers each): at most eight, made as
+// they are needed.
+struct SlotPool;
 
-// A scene came to the calling thread's current context, or left the context so
-// named: the last one to leave gives the buffers kept for its queries back. They
-// are kept in a device's primary context alone; elsewhere a call has its own, and
-// there is nothing to release.
-std::optional<std::uint64_t> retainQueryBuffers();
-void releaseQueryBuffers(std::uint64_t context);
+// A scene came to the calling thread's current context: the slots kept for queries
+// there, until the last scene leaves it. They are kept in a device's primary
+// context alone; a context that a program made may be destroyed while scenes of it
+// are alive, and its streams with it. Null elsewhere: a call has its own.
+SlotPool* retainQueryBuffers();
+void releaseQueryBuffers(SlotPool* kept);
+
+// Runs `count` queries in the calling thread's current context, that of the scene
+// that holds `kept`, after the work that the default stream held when the call was
+// made, and returns when every result is in its host array. Safe from several
+// threads. Throws std::bad_alloc, or std::runtime_error for any other CUDA failure.
+void runQueries(SlotPool* kept, std::int64_t count, std::span<const QueryInput> inputs,
+                std::span<const QueryOutput> outputs, const QueryLaunch& launch);
 
 } // namespace albedo_b200

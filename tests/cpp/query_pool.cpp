@@ -237,6 +237,8 @@ cudaError_t twicePlusOne(void* const* in, void* const* out, int count, cudaStrea
     return cudaGetLastError(); // as a launch reports what went wrong before it
 }
 
+SlotPool* kept = nullptr; // of the scene that main() holds
+
 std::vector<int> numbers(std::size_t count)
 {
     std::vector<int> v(count);
@@ -259,7 +261,7 @@ void run(const std::vector<int>& in, std::vector<int>& out)
 {
     const QueryInput inputs[]{{in.data(), sizeof(int)}};
     const QueryOutput outputs[]{{out.data(), sizeof(int)}};
-    runQueries(static_cast<std::int64_t>(in.size()), inputs, outputs, twicePlusOne);
+    runQueries(kept, static_cast<std::int64_t>(in.size()), inputs, outputs, twicePlusOne);
 }
 
 // Inputs that work on the default stream is still to fill when the call is made.
@@ -282,9 +284,13 @@ void context()
 {
     for (const std::uintptr_t own : {1, 7, 1}) {
         fake::current = own;
+        SlotPool* const before = kept;
+        kept = retainQueryBuffers();
         const std::vector<int> in = numbers(300'007);
         std::vector<int> out(in.size(), 5);
         run(in, out);
+        releaseQueryBuffers(kept);
+        kept = before;
         std::printf("context own=%d after=%d wrong=%zu elsewhere=%d kept_elsewhere=%d\n", static_cast<int>(own),
                     static_cast<int>(fake::current), wrongAnswers(in, out.data()), fake::used_elsewhere.load(),
                     [] {
@@ -304,11 +310,10 @@ void scenes()
     const std::vector<int> in = numbers(300'007);
     std::vector<int> out(in.size(), 5);
     run(in, out);
-    const auto share = retainQueryBuffers();
-    releaseQueryBuffers(*share);
-    const std::size_t kept = fake::alive();
+    releaseQueryBuffers(retainQueryBuffers());
+    const bool still = fake::alive() > 0;
     fake::current = 7;
-    std::printf("scenes kept=%d own_share=%d\n", kept > 0 ? 1 : 0, retainQueryBuffers() ? 1 : 0);
+    std::printf("scenes kept=%d own_share=%d\n", still ? 1 : 0, retainQueryBuffers() != nullptr ? 1 : 0);
 }
 
 // Device memory for nothing, for a small slot, for one slot and for three of those
@@ -345,7 +350,7 @@ void overlap()
                 int* const results = both.data() + behind;
                 const QueryInput inputs[]{{both.data() + before, sizeof(int)}};
                 const QueryOutput outputs[]{{results, sizeof(int)}};
-                runQueries(static_cast<std::int64_t>(count), inputs, outputs, twicePlusOne);
+                runQueries(kept, static_cast<std::int64_t>(count), inputs, outputs, twicePlusOne);
                 std::printf("overlap count=%zu wrong=%zu\n", count, wrongAnswers(in, results));
             }
         }
@@ -353,7 +358,7 @@ void overlap()
         std::vector<int> both(4 * count);
         const QueryInput inputs[]{{in.data(), sizeof(int)}};
         const QueryOutput outputs[]{{both.data() + 3 * count - count / 2, sizeof(int)}, {both.data(), 3 * sizeof(int)}};
-        runQueries(static_cast<std::int64_t>(count), inputs, outputs,
+        runQueries(kept, static_cast<std::int64_t>(count), inputs, outputs,
                    [](void* const* i, void* const* o, int n, cudaStream_t stream) {
                        for (int k = 0; k < 3 * n; ++k) {
                            static_cast<int*>(o[1])[k] = -7;
@@ -382,9 +387,9 @@ int main(int argc, char** argv)
     if (check == checks.end()) {
         return 2;
     }
-    const auto share = retainQueryBuffers();
+    kept = retainQueryBuffers();
     check->second();
-    releaseQueryBuffers(*share);
+    releaseQueryBuffers(kept);
     std::printf("end left=%zu\n", fake::alive());
     return 0;
 }
