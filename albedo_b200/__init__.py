@@ -430,17 +430,19 @@ def autotune_batch(items) -> dict:
 def set_tuning(scene: Scene | None = None, **shape) -> None:
     """Pins a launch shape: tile_width, blocks_per_sm and inline_traversal for a scene's megakernel,
     or (no scene) blocks_per_sm, trace_blocks_per_sm, fetch_batch, trace_loop, ray_sort,
-    iterations_per_graph and slot_count for the wavefront engine."""
+    iterations_per_graph and slot_count for the wavefront engine. For a scene it takes what
+    tuning(scene) returned whole: that of a scene without a shape (evaluations -1) leaves it without one."""
     t = TuningC()
     for k, v in shape.items():
-        if k not in _TUNING_FIELDS[:9]:
+        if k not in _TUNING_FIELDS:
             raise ValueError(f"unknown shape field {k}")
-        setattr(t, k, int(v))
+        setattr(t, k, v if k in ("best_ms", "default_ms") else int(v))
     _raise(library().albedo_tuning_set(None if scene is None else scene.handle, byref(t)))
 
 
 def tuning(scene: Scene | None = None) -> dict:
-    """The shape renders use now: the scene's megakernel shape, or (no scene) the wavefront engine's."""
+    """The shape renders use now: the scene's megakernel shape (evaluations -1 if it has none of its own and
+    each launch chooses), or (no scene) the wavefront engine's."""
     out = TuningC()
     _raise(library().albedo_tuning_get(None if scene is None else scene.handle, byref(out)))
     return _tuning_dict(out)

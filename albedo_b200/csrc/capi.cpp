@@ -1315,6 +1315,13 @@ int albedo_autotune_batch(const albedo_batch_item* items, int32_t count, albedo_
     });
 }
 
+namespace {
+
+// `evaluations` of a megakernel shape that was read from a scene without one of its own.
+constexpr int32_t kNoShape{-1};
+
+} // namespace
+
 int albedo_tuning_set(albedo_scene* scene, const albedo_tuning* shape)
 {
     return guarded([&] {
@@ -1332,9 +1339,10 @@ int albedo_tuning_set(albedo_scene* scene, const albedo_tuning* shape)
                 throw std::invalid_argument{"megakernel traversal placement must be 0 (out of line), 1 (inlined) or "
                                             "2 (closest hit inlined, 3 blocks per SM only)"};
             }
-            scene->mega_tile_width = shape->tile_width;
-            scene->mega_blocks_per_sm = shape->blocks_per_sm;
-            scene->mega_inline = shape->inline_traversal;
+            const bool own{shape->evaluations != kNoShape};
+            scene->mega_tile_width = own ? shape->tile_width : 0;
+            scene->mega_blocks_per_sm = own ? shape->blocks_per_sm : 0;
+            scene->mega_inline = own ? shape->inline_traversal : 0;
             return;
         }
         if (shape->blocks_per_sm <= 0 || shape->trace_blocks_per_sm <= 0 || shape->fetch_batch <= 0 ||
@@ -1371,6 +1379,7 @@ int albedo_tuning_get(const albedo_scene* scene, albedo_tuning* out)
             out->tile_width = scene->mega_tile_width > 0 ? scene->mega_tile_width : 16;
             out->blocks_per_sm = scene->mega_blocks_per_sm > 0 ? scene->mega_blocks_per_sm : 3;
             out->inline_traversal = scene->mega_inline;
+            out->evaluations = scene->mega_blocks_per_sm > 0 ? 0 : kNoShape;
             return;
         }
         const std::lock_guard lock{g_engine_mutex};

@@ -334,7 +334,8 @@ typedef struct albedo_tuning {
     int32_t fetch_batch;          /* wavefront: queue entries a traversal warp claims at once */
     int32_t iterations_per_graph; /* wavefront: iterations per captured CUDA graph */
     int32_t slot_count;           /* wavefront: path slots */
-    int32_t evaluations;          /* shapes timed */
+    int32_t evaluations;          /* shapes timed; -1 from albedo_tuning_get for a scene without a shape
+                                     of its own */
     int32_t inline_traversal;     /* megakernel: 0 = one out-of-line traversal copy serves both queries,
                                      1 = both queries' traversal inlined into the kernel, 2 = the
                                      closest-hit query's inlined and the shadow query's out of line
@@ -360,14 +361,18 @@ int albedo_autotune_megakernel(albedo_scene* scene, const albedo_render_job* job
  * the process. */
 int albedo_autotune_batch(const albedo_batch_item* items, int32_t count, albedo_tuning* out);
 /* The shape renders use now: the scene's megakernel shape (scene not NULL) or
- * the process's wavefront shape (scene NULL); timing fields are zero. */
+ * the process's wavefront shape (scene NULL). Timing fields are zero, but for
+ * evaluations, which is -1 for a scene without a shape of its own: each launch
+ * then chooses, and the fields are those of an image of medium size. */
 int albedo_tuning_get(const albedo_scene* scene, albedo_tuning* out);
 /* Pins a shape, as the autotuner would keep it: the scene's megakernel shape
  * (scene not NULL: tile_width 8, 16 or 32, blocks_per_sm 3 or 4, and
  * inline_traversal 0, 1 or 2, the last with 3 blocks per SM) or the
  * process's wavefront shape (scene NULL: blocks_per_sm, trace_blocks_per_sm,
  * fetch_batch, iterations_per_graph and slot_count, all positive, and
- * trace_loop 0, 1 or 2, ray_sort 0, 1 or 2). Timing fields are ignored. Images do not depend on the
+ * trace_loop 0, 1 or 2, ray_sort 0, 1 or 2). Timing fields are ignored, but for
+ * evaluations -1 with a scene, which takes the scene's shape away: what
+ * albedo_tuning_get wrote can be set again whole. Images do not depend on the
  * shape. */
 int albedo_tuning_set(albedo_scene* scene, const albedo_tuning* shape);
 /* Iterations the last wavefront run took. */
