@@ -381,23 +381,36 @@ cudaError_t chooseWarpPixels(const DevScene& scene, RenderArgs& args)
 // scatter between 0.92 and 1.08 at 800x450.
 constexpr int kDefaultWarpsPerSm = kMegaBlocksPerSm * kBlock / 32;
 
+constexpr int defaultBlocksPerSm(long long pixels, int sms, int warp_pixels, float mesh_steps)
+{
+    constexpr int kManyWaves = 20;
+    constexpr int kCostlyMeshWaves = 6;
+    constexpr float kCostlyMeshSteps = 40.0f;
+    const int waves = mesh_steps >= kCostlyMeshSteps ? kCostlyMeshWaves : kManyWaves;
+    const long long full = static_cast<long long>(sms) * kDefaultWarpsPerSm * warp_pixels * waves;
+    return pixels >= full ? 4 : kMegaBlocksPerSm;
+}
+
+// Both sides of each limit, for 148 SMs (12 x 32 x 148 = 56,832 pixels a wave).
+static_assert(kMegaBlocksPerSm != 3 ||
+              (defaultBlocksPerSm(20 * 56832 - 1, 148, 32, 39.9f) == 3 &&
+               defaultBlocksPerSm(20 * 56832, 148, 32, 0.0f) == 4 &&
+               defaultBlocksPerSm(6 * 56832 - 1, 148, 32, 40.0f) == 3 &&
+               defaultBlocksPerSm(6 * 56832, 148, 32, 40.0f) == 4 &&
+               defaultBlocksPerSm(6 * 56832, 148, 32, 39.9f) == 3 && defaultBlocksPerSm(1, 148, 1, 200.0f) == 3));
+
 cudaError_t chooseBlocksPerSm(RenderArgs& args)
 {
     if (args.blocks_per_sm != 0 || args.estimator != kEstimatorPath) {
         return cudaSuccess;
     }
-    constexpr int kManyWaves = 20;
-    constexpr int kCostlyMeshWaves = 6;
-    constexpr float kCostlyMeshSteps = 40.0f;
-    const int waves = args.mesh_steps >= kCostlyMeshSteps ? kCostlyMeshWaves : kManyWaves;
     int device = 0;
     int sms = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e == cudaSuccess) {
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     }
-    const long long full = static_cast<long long>(sms) * kDefaultWarpsPerSm * args.warp_pixels * waves;
-    args.blocks_per_sm = imagePixels(args) >= full ? 4 : kMegaBlocksPerSm;
+    args.blocks_per_sm = defaultBlocksPerSm(imagePixels(args), sms, args.warp_pixels, args.mesh_steps);
     return e;
 }
 
