@@ -337,9 +337,8 @@ double halfArea(double x, double y, double z)
     return x * y + y * z + z * x;
 }
 
-// Nodes of nodes[first ..] a line through the root's box is expected to enter: a
-// uniformly random line that enters a convex body enters a box inside it with the
-// ratio of their surface areas (Goldsmith and Salmon 1987).
+} // namespace
+
 float expectedNodeSteps(const std::vector<DevNode>& nodes, std::size_t first, std::uint32_t root)
 {
     if (first == nodes.size() || root == kEmptyChild) {
@@ -362,8 +361,6 @@ float expectedNodeSteps(const std::vector<DevNode>& nodes, std::size_t first, st
     }
     return whole > 0.0 ? static_cast<float>(1.0 + sum / whole) : 0.0f;
 }
-
-} // namespace
 
 DeviceImage flattenScene(const HostScene& scene)
 {

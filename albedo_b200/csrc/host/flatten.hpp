@@ -39,6 +39,12 @@ struct DeviceImage {
     float mesh_steps{0.0f};
 };
 
+// Nodes of nodes[first ..] a line through the box of the mesh they hold, whose root
+// is nodes[root], is expected to enter: a uniformly random line that enters a convex
+// body enters a box inside it with the ratio of their surface areas (Goldsmith and
+// Salmon 1987). Zero for a mesh without triangles.
+float expectedNodeSteps(const std::vector<DevNode>& nodes, std::size_t first, std::uint32_t root);
+
 // Throws std::invalid_argument if the scene exceeds the device layout's limits
 // (leaf positions must fit 28 bits), and LayoutLimitError if a coordinate of
 // its geometry, instance maps or lights is beyond FP32's range.
