@@ -27,6 +27,8 @@ L2 read peak measured in the same run by a read sweep of this library.
 this machine's host cores rendering the same frame through its own renderImage
 at 36 samples per pixel. `precision` holds every form's error on this frame
 against the FP64 oracle (the reference at 65,536 spp on 2,048 seeded pixels).
+Where the reference renderer can be neither found nor built, `--impl reference`
+prints a line that says so, and so do these two in place of their figures.
 
 `forms` (1 GPU, unless --no-forms) adds the other configurations: the 1M-triangle
 random soup at the same frame; the instanced trefoil frame (960x540, 64 spp),
@@ -270,6 +272,15 @@ def profiled_traffic(name: str, paths: int) -> tuple[float | None, str | None]:
 # ------------------------------------------------------------------ the reference on the host
 
 
+def reference_missing() -> str | None:
+    """Why the reference renderer cannot be run here, or None if it can."""
+    from oracle import reference as ref
+
+    if ref.available():
+        return None
+    return "the reference renderer's library is not here and its sources, to build it from, are absent"
+
+
 def reference_frame_sample(scene_path: Path, frame: Frame, samples_per_axis: int = REFERENCE_SAMPLES_PER_AXIS,
                            scene=None) -> dict:
     """The reference's own renderImage on the full frame of `frame` at
@@ -295,6 +306,10 @@ def run_reference(args, rank: int) -> None:
     rendering the headline frame through renderImage on the host's cores; each
     step is the full frame at 16 spp."""
     if rank != 0:
+        return
+    missing = reference_missing()
+    if missing is not None:
+        print(json.dumps({"impl": "reference", "unavailable": missing}), flush=True)
         return
     from albedo_b200 import scenes
     from oracle import reference as ref
@@ -336,6 +351,9 @@ def precision_errors(scene_path: Path, frame: Frame, images: dict, pixel_count: 
     luminance exceeds 1e-3, and the paired statistic of each image's per-pixel
     squared errors against the reference's (mean difference over its standard
     error: |t| < 4 is matched RMSE)."""
+    missing = reference_missing()
+    if missing is not None:
+        return {"unavailable": missing}
     from oracle import reference as ref
 
     rng = np.random.default_rng(91)
@@ -957,7 +975,9 @@ def main():
             "autotune": tuned,
         }
         if world == 1:
-            line["cpu_baseline"] = reference_frame_sample(scene_path, frame, BASELINE_SAMPLES_PER_AXIS)
+            missing = reference_missing()
+            line["cpu_baseline"] = ({"unavailable": missing} if missing is not None
+                                    else reference_frame_sample(scene_path, frame, BASELINE_SAMPLES_PER_AXIS))
             if not args.no_forms and method == ab.MEGAKERNEL:
                 accum.zero_()
                 ab.render_device(scene, job, accum.data_ptr())
