@@ -170,6 +170,9 @@ struct SlotPool {
     std::size_t made{0};
     int scenes{0};
 
+    // Slots are put back from destructors, which must not allocate.
+    SlotPool() { idle.reserve(kMaxWorkers); }
+
     // A slot for the caller of a query: waits for one while all are in use, and
     // takes a small one where there is no memory for a whole one.
     std::unique_ptr<Slot> take()
@@ -489,14 +492,15 @@ void releaseQueryBuffers(SlotPool* kept)
     if (kept == nullptr) {
         return;
     }
-    std::vector<std::unique_ptr<Slot>> given;
+    std::array<std::unique_ptr<Slot>, kMaxWorkers> given;
     {
         const std::lock_guard lock{kept->mutex};
         if (--kept->scenes > 0) {
             return;
         }
-        given.swap(kept->idle);
-        kept->made -= given.size();
+        std::move(kept->idle.begin(), kept->idle.end(), given.begin());
+        kept->made -= kept->idle.size();
+        kept->idle.clear();
         kept->freed.notify_all();
     }
 }
