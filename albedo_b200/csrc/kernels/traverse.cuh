@@ -583,7 +583,7 @@ ALB_DEV unsigned loadEntry(const TraceStack<unsigned>&, unsigned at)
 // that part, but each axis's origin and inverse take a register pair. The path
 // estimator's megakernel (168 registers a thread) gains, ms: trefoils 277.6 ->
 // 270.4, icosphere 181.7 -> 179.9, soup 49.2 -> 48.8, sphere room 8.42 -> 8.24.
-// The others lose and keep the scalar form: the scatter-only estimator (140
+// The others lose and keep the scalar form: the scatter-only estimator (136
 // registers) 172.2 -> 174.4 in the room at 1174x843, the persistent kernels (96)
 // 51.0 -> 51.4 for the trefoils.
 template <bool PACKED, typename Stack>

@@ -61,7 +61,8 @@ ALB_DEV unsigned long long claimItem(unsigned long long* next, bool want)
 }
 
 // Resident blocks per SM the traversal kernels' register budget is sized for:
-// 5 (96 registers a thread, tens of bytes of spills). With 4-byte stack entries five blocks'
+// 5 (96 registers a thread; with a step a turn the extend kernel spills 40 bytes and
+// reloads 96, the shadow kernel 36 of each). With 4-byte stack entries five blocks'
 // stacks fit in shared memory; 5 measured 6-10% faster than 4 on the trefoil,
 // icosphere and 64-job workloads.
 #ifndef ALBEDO_TRACE_BLOCKS_PER_SM
@@ -343,11 +344,13 @@ ALB_DEV int raysPerWarp(int count)
 // dependent memory accesses whatever the number of lanes, and most single steps
 // end the query of only one or two. Once the queue is empty the warp finishes
 // what it holds.
-// Measured against the whole query a turn (fetches of 32 rays), ms: instanced
-// trefoils 960x540 at 16 samples 58.2 -> 54.4, 81,920-triangle icosphere 36.5 ->
-// 34.2, 200,003-triangle soup 853x481 80.2 -> 72.2, 16-job batch 124.5 -> 120.7;
-// filing after every step 60.4 / 38.3 / 79.3 / 137.2. Thresholds of 8 to 24 lanes
-// are within 1% of 16, and fetches of 16 rays beat 32 by 2-5% and 64 by far.
+// Measured when it was taken against the whole query a turn, ms: instanced trefoils
+// 960x540 at 16 samples 58.2 -> 54.4, 81,920-triangle icosphere 36.5 -> 34.2,
+// 200,003-triangle soup 853x481 80.2 -> 72.2, 16-job batch 124.5 -> 120.7; filing
+// after every step 60.4 / 38.3 / 79.3 / 137.2. Thresholds of 8 to 24 lanes are
+// within 1% of 16. Fetches of 32 rays, the default, now give 46.8 / 29.0 / 66.0 /
+// 101.8; of 16 rays 47.1 / 28.7 / 66.3 / 101.7, of 8 48.0 / 28.8 / 66.3 / 103.6, of
+// 64 50.1 / 30.5 / 68.9 / 107.2.
 template <int LOOP>
 ALB_DEV bool traceWarp(const DevScene* scene, TraceState& q, const SkipRule& skip, const TraceStack<unsigned>& stack,
                        unsigned int* error_flag, bool any, bool drained, int lanes, bool& active)
