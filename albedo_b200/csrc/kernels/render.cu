@@ -378,7 +378,10 @@ cudaError_t chooseWarpPixels(const DevScene& scene, RenderArgs& args)
 // waves: 0.89 to 1.05; 640x360, 4 waves: up to 1.11. Soups of 20,000 to 300,000
 // triangles (mesh_steps 43 to 221) take 0.80 to 0.92 from 800x450, 6.3 waves, on,
 // but up to 1.06 at 640x360. Closed surfaces of 1,280 to 1.31M triangles (12 to 24)
-// scatter between 0.92 and 1.08 at 800x450.
+// scatter between 0.92 and 1.08 at 800x450. The costliest mesh decides, however small:
+// soups of 20,000 and 200,000 triangles and a tenth to half the size of the trefoils
+// or the icosphere beside them take 0.92 to 0.99 from 800x450 on; beside the
+// icosphere and as large as it, 1.10 at 800x450 and 0.94 to 0.99 at 960x540.
 constexpr int kDefaultWarpsPerSm = kMegaBlocksPerSm * kBlock / 32;
 
 constexpr int defaultBlocksPerSm(long long pixels, int sms, int warp_pixels, float mesh_steps)

@@ -12,8 +12,8 @@
 // the reference's byte exactly and the kernel evaluates no power function; and
 // where a quotient good to 2^-44 is not next to a decision it stands for the
 // exact one. A pure stream: 32 bytes read and 3 written per pixel, the reads as
-// one coalesced 256-bit load per pixel; 3840x2160 takes 51.5 us, 86% of the
-// measured copy bandwidth.
+// one coalesced 256-bit load per pixel; 3840x2160 takes 51.6 us among other
+// launches, 86% of the measured copy bandwidth, and 54.3 by itself.
 #include "launch.hpp"
 
 #include <algorithm>
@@ -26,8 +26,8 @@ namespace {
 // The tiled kernel: one block of 24 warps per SM, four pixels a lane in flight
 // (4 KB a warp, 96 KB an SM). Every block packs the tables into shared memory
 // first, from constant-bank reads that differ per lane, so fewer and wider
-// blocks start sooner: 3840x2160 51.5 us, against 55.7 for four blocks of 256
-// threads and 67.8 for eight (1920x1080 18.5, 24.0 and 30.8).
+// blocks start sooner: among other launches 3840x2160 51.6 us, against 55.7 for four
+// blocks of 256 threads and 67.8 for eight (1920x1080 18.5, 24.0 and 30.8).
 constexpr int kTileThreads{768};
 constexpr int kTileBlocksPerSm{1};
 constexpr int kResolveGroup{4};

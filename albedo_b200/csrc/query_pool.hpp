@@ -10,9 +10,9 @@
 // allocated after the first calls.
 // Measured on 16 host cores, from and to pageable arrays, instanced trefoils, ms
 // (pageable copies and per-call buffers -> this): 1,000,003 any-hit queries 4.89
-// -> 1.61, 1,000 of them 0.13 -> 0.08, 262,144 closest hits with their geometry
-// 7.37 -> 2.38, 1,048,576 without 8.09 -> 2.68. The first call of a size pays
-// about a millisecond for each worker's buffers.
+// -> 1.61, 1,000 of them 0.13 -> 0.07; closest hits with their geometry 262,144
+// 7.37 -> 2.38, 10,000 0.385 -> 0.180, 100 0.200 -> 0.092; 1,048,576 without 8.09 ->
+// 2.68. The first call of a size pays about a millisecond for each worker's buffers.
 #pragma once
 
 #include <cuda_runtime_api.h>
