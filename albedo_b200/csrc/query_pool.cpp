@@ -358,8 +358,8 @@ bool arraysOverlap(std::size_t count, std::span<const QueryInput> inputs, std::s
 // A call whose outputs lie over its inputs or each other reads every input before
 // it writes a result and writes its outputs whole, one after the other; its chunks,
 // which run beside each other, work on copies.
-void runOnCopies(SlotPool* kept, std::int64_t count, std::span<const QueryInput> inputs, std::span<const QueryOutput> outputs,
-                 const QueryLaunch& launch)
+void runOnCopies(SlotPool* kept, std::int64_t count, std::span<const QueryInput> inputs,
+                 std::span<const QueryOutput> outputs, const QueryLaunch& launch)
 {
     const auto n{static_cast<std::size_t>(count)};
     std::vector<std::vector<char>> memory;
