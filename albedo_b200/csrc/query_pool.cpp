@@ -277,12 +277,7 @@ SlotPool& keptSlots(std::uint64_t context)
 class HeldSlot {
 public:
     HeldSlot(SlotPool& pool, std::unique_ptr<Slot> slot) : pool_{pool}, slot_{std::move(slot)} {}
-    // A worker that failed may leave copies in flight that use the buffers.
-    ~HeldSlot()
-    {
-        cudaStreamSynchronize(slot_->stream);
-        pool_.give(std::move(slot_));
-    }
+    ~HeldSlot() { pool_.give(std::move(slot_)); }
     HeldSlot(const HeldSlot&) = delete;
     HeldSlot& operator=(const HeldSlot&) = delete;
     Slot& operator*() const { return *slot_; }
@@ -422,8 +417,15 @@ void runQueries(SlotPool* kept, std::int64_t count, std::span<const QueryInput> 
         for (std::int64_t c{next++}; c < chunks; c = next++) {
             const std::int64_t end{std::min((c + 1) * chunk, count)};
             for (std::int64_t first{c * chunk}; first < end; first += slot.rays) {
-                runChunk(slot, static_cast<std::size_t>(first),
-                         static_cast<std::size_t>(std::min(slot.rays, end - first)), inputs, outputs, launch);
+                const std::int64_t n{std::min(slot.rays, end - first)};
+                try {
+                    runChunk(slot, static_cast<std::size_t>(first), static_cast<std::size_t>(n), inputs, outputs,
+                             launch);
+                } catch (...) {
+                    // What failed may have left copies in flight that use the buffers.
+                    cudaStreamSynchronize(slot.stream);
+                    throw;
+                }
             }
         }
     };

@@ -19,6 +19,7 @@
 #include <map>
 #include <mutex>
 #include <new>
+#include <stdexcept>
 #include <string>
 #include <vector>
 
@@ -80,6 +81,24 @@ void use(const void* p)
     if (found == made.begin() || (--found)->second.context != useCurrent()) {
         ++used_elsewhere;
     }
+}
+// Copies and clears on each stream since something last waited for it.
+std::map<cudaStream_t, int> pending;
+
+void enqueue(cudaStream_t stream)
+{
+    use(stream);
+    const std::lock_guard lock{mutex};
+    ++pending[stream];
+}
+int inFlight()
+{
+    const std::lock_guard lock{mutex};
+    int n = 0;
+    for (const auto& [stream, count] : pending) {
+        n += count;
+    }
+    return n;
 }
 std::size_t alive()
 {
@@ -197,6 +216,8 @@ cudaError_t cudaStreamSynchronize(cudaStream_t stream)
         fake::default_stream.clear();
     } else {
         fake::use(stream);
+        const std::lock_guard lock{fake::mutex};
+        fake::pending[stream] = 0;
     }
     return cudaSuccess;
 }
@@ -204,14 +225,14 @@ cudaError_t cudaMemcpyAsync(void* to, const void* from, size_t bytes, cudaMemcpy
 {
     fake::use(to);
     fake::use(from);
-    fake::use(stream);
+    fake::enqueue(stream);
     std::memcpy(to, from, bytes);
     return cudaSuccess;
 }
 cudaError_t cudaMemsetAsync(void* to, int value, size_t bytes, cudaStream_t stream)
 {
     fake::use(to);
-    fake::use(stream);
+    fake::enqueue(stream);
     std::memset(to, value, bytes);
     return cudaSuccess;
 }
@@ -377,12 +398,36 @@ void overlap()
     }
 }
 
+// Launches that fail, the first, a later one and all of them; then a call that does not.
+void failure()
+{
+    const std::vector<int> in = numbers(300'007);
+    for (const int bad : {0, 5, -1, 1000}) {
+        std::vector<int> out(in.size(), 5);
+        const QueryInput inputs[]{{in.data(), sizeof(int)}};
+        const QueryOutput outputs[]{{out.data(), sizeof(int)}};
+        std::atomic<int> launches{0};
+        bool failed = false;
+        try {
+            runQueries(kept, static_cast<std::int64_t>(in.size()), inputs, outputs,
+                       [&](void* const* i, void* const* o, int n, cudaStream_t stream) {
+                           const int k = launches++;
+                           return k == bad || bad < 0 ? cudaErrorLaunchFailure : twicePlusOne(i, o, n, stream);
+                       });
+        } catch (const std::runtime_error&) {
+            failed = true;
+        }
+        std::printf("failure bad=%d failed=%d flight=%d wrong=%zu\n", bad, failed ? 1 : 0, fake::inFlight(),
+                    failed ? std::size_t{0} : wrongAnswers(in, out.data()));
+    }
+}
+
 } // namespace
 
 int main(int argc, char** argv)
 {
     const std::map<std::string, void (*)()> checks{{"order", order}, {"context", context}, {"scenes", scenes},
-                                                      {"memory", memory}, {"overlap", overlap}};
+                                                      {"memory", memory}, {"overlap", overlap}, {"failure", failure}};
     const auto check = checks.find(argc > 1 ? argv[1] : "");
     if (check == checks.end()) {
         return 2;

@@ -59,3 +59,8 @@ def test_a_call_runs_with_the_buffers_there_is_memory_for(exe):
 def test_outputs_over_other_arrays_are_written_after_they_are_read(exe):
     found = findings(exe, "overlap")
     assert len(found) == 30 and all(f["wrong"] == 0 for f in found), found
+
+
+def test_a_call_that_fails_leaves_nothing_in_flight(exe):
+    assert findings(exe, "failure") == [{"bad": bad, "failed": int(bad < 1000), "flight": 0, "wrong": 0}
+                                        for bad in (0, 5, -1, 1000)]
